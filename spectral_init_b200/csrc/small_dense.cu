@@ -18,6 +18,7 @@
 // The Gram matrices come from the fused device pass over the blocks, so the
 // residuals never need an explicit orthogonalisation pass.
 #include <cfloat>
+#include <cstddef>
 #include <cstdlib>
 #include <string>
 
@@ -36,6 +37,7 @@ struct SmallSmem {
   double* Z;
   double* T;  // second buffer of A for the double-buffered Jacobi
   int ld;
+  double* W;  // scratch of cta_tri_select (kTriWork doubles; parallel form only)
 };
 
 // Sweep stopping test of the Jacobi eigensolvers: the off-diagonal Frobenius
@@ -778,122 +780,519 @@ __device__ bool warp_rr_general(const double* gb, const double* ga, int P, const
   return true;
 }
 
-// The generalised Rayleigh-Ritz of cta_rr_general with its serial sections
-// made parallel: the D-scale factors one per thread; a right-looking
-// Cholesky with one barrier per pivot (every thread recomputes the pivot, the
-// trailing update reads the unscaled pivot column, and the column scaling is
-// one pass at the end); L^-1 formed once, one column per thread, so that
-// C = L^-1 A L^-T and the Ritz vectors D L^-T V_sel are parallel matrix
-// products instead of three one-thread-per-column triangular solves; the
-// selection order by ranks.  Same results as cta_rr_general up to rounding.
-__device__ bool cta_rr_general_par(const double* gb, const double* ga, int P, const int* idx, int s, int nsel,
-                                   int largest, double chol_tol, SmallSmem sm, double* dsc, double* theta_out,
-                                   double* red, int* order, int* sflag) {
-  __shared__ double lsq[3 * MAXM];  // sqrt of the pivots, then 1 / L_jj
-  const int ld = sm.ld;
-  const int nt = blockDim.x;
-  if (threadIdx.x == 0) *sflag = 0;
-  for (int t = threadIdx.x; t < s * s; t += nt) {
-    const int i = t / s, j = t % s;
-    sm.B[i * ld + j] = gb[idx[i] * P + idx[j]];
-    sm.A[i * ld + j] = ga[idx[i] * P + idx[j]];
+// ---------------------------------------------------------------------------
+// The nsel smallest (largest) eigenpairs of a symmetric s x s matrix, s <= 48,
+// by the direct route: Householder tridiagonalisation, multisection of the
+// wanted eigenvalues (one warp each), eigenvectors from twisted
+// factorisations of T - theta (Parlett and Dhillon, "Fernando's solution to
+// Wilkinson's problem", LAA 267, 1997), a symmetric (Newton-Schulz)
+// orthonormalisation and the back-transformation.  The Rayleigh-Ritz step
+// wants at most a third of the pairs, and a cyclic Jacobi pays about four
+// sweeps of s - 1 two-barrier rounds for all of them: the chain here is s - 2
+// reflectors, 11 counts and one factorisation long.  Measured (whole small
+// step, B200): 12 x 12 49 -> SMALL12 us, 48 x 48 493 -> SMALL48 us.
+//
+// The result is backward stable (a computed vector is off by eps / gap along
+// a neighbour, which moves the projected matrix by eps) unless two wanted
+// eigenvalues agree to about 1e-14 of the norm; then the vectors come out
+// nearly parallel, the orthonormality or the residual test fails and false is
+// returned: the caller falls back to the Jacobi iteration.
+//   A (ld): destroyed (rows keep the reflectors); V (ld): s x nsel vectors;
+//   work: kTriWork doubles, 16-byte aligned; theta: nsel values, ascending (descending for
+//   `largest`).
+constexpr int kTriMax = 3 * MAXM;
+constexpr int kTriWarps = 16;  // warps that take an eigenpair each
+constexpr int kTriWork = kTriWarps * 4 * kTriMax;  // doubles of scratch
+
+// Householder tridiagonalisation.  Lane l owns columns l and l + 32; the rows
+// of the symmetric matrix are split over the engaged warps (one, without
+// barriers, up to 16 columns; four above, where more warps only re-read the
+// partial products: 16 warps cost 3.3 k cycles a column at 48 x 48).  Every
+// engaged warp forms the reflector and w redundantly, so a column costs two
+// barriers.  H = I - tau v v^T with v_{j+1} = alpha - beta unnormalised: the
+// one division, tau = 1 / (beta (beta - alpha)), overlaps the product A v.
+__device__ __forceinline__ void hh_barrier(bool multi) {
+  if (multi) asm volatile("bar.sync 1, 128;" ::: "memory");
+  else __syncwarp();
+}
+
+__device__ __forceinline__ double warp_sum_low(double v, bool half) {
+  // lanes 16..31 hold zero when half: one level less
+  if (!half) v += __shfl_xor_sync(0xffffffffu, v, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+__device__ void cta_householder(double* A, int s, int ld, double* d, double* e, double* tau, double* vs, double* ws,
+                                double* part, bool multi) {
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int nw = multi ? 4 : 1;
+  if (warp >= nw) return;
+  const int l1 = lane + 32;
+  const bool wide = s > 32;
+  const bool half = s <= 16;
+  for (int j = 0; j + 2 < s; ++j) {
+    const double* row = A + j * ld;
+    double x0 = (lane > j && lane < s) ? row[lane] : 0.0;
+    double x1 = (wide && l1 > j && l1 < s) ? row[l1] : 0.0;
+    const double alpha = row[j + 1];
+    const double diag = row[j];
+    double sq = lane == j + 1 ? 0.0 : x0 * x0;
+    if (l1 != j + 1) sq = fma(x1, x1, sq);
+    // half: the sum is over lanes 0..15 and read back from lane 0's half
+    double sigma = warp_sum_low(sq, half);
+    if (half) sigma = __shfl_sync(0xffffffffu, sigma, 0);
+    double t = 0.0, beta = alpha;
+    if (sigma > 0.0) {
+      const double nrm = sqrt(fma(alpha, alpha, sigma));
+      beta = alpha >= 0.0 ? -nrm : nrm;
+      t = beta * (beta - alpha);  // its reciprocal below
+      if (lane == j + 1) x0 = alpha - beta;
+      if (l1 == j + 1) x1 = alpha - beta;
+    } else {
+      x0 = 0.0;
+      x1 = 0.0;
+    }
+    // the same values from every engaged warp; rewritten only after the barrier that ends the column
+    if (lane < s) vs[lane] = x0;
+    if (wide && l1 < s) vs[l1] = x1;
+    __syncwarp();
+    if (t != 0.0) {
+      t = 1.0 / t;
+      double p0 = 0.0, p1 = 0.0, r0 = 0.0, r1 = 0.0;
+      int k = j + 1 + warp;
+      const int c0 = min(lane, s - 1), c1 = wide ? min(l1, s - 1) : 0;
+      for (; k + nw < s; k += 2 * nw) {
+        const double va = vs[k], vb = vs[k + nw];
+        p0 = fma(A[k * ld + c0], va, p0);
+        r0 = fma(A[(k + nw) * ld + c0], vb, r0);
+        if (wide) {
+          p1 = fma(A[k * ld + c1], va, p1);
+          r1 = fma(A[(k + nw) * ld + c1], vb, r1);
+        }
+      }
+      if (k < s) {
+        p0 = fma(A[k * ld + c0], vs[k], p0);
+        if (wide) p1 = fma(A[k * ld + c1], vs[k], p1);
+      }
+      p0 += r0;
+      p1 += r1;
+      if (multi) {
+        part[warp * kTriMax + lane] = p0;
+        if (l1 < kTriMax) part[warp * kTriMax + l1] = p1;
+        hh_barrier(true);
+        p0 = (part[lane] + part[kTriMax + lane]) + (part[2 * kTriMax + lane] + part[3 * kTriMax + lane]);
+        if (l1 < kTriMax)
+          p1 = (part[l1] + part[kTriMax + l1]) + (part[2 * kTriMax + l1] + part[3 * kTriMax + l1]);
+      }
+      p0 *= t;
+      p1 *= t;
+      // x is zero outside columns j + 1 .. s - 1
+      double h = warp_sum_low(fma(p0, x0, p1 * x1), half);
+      if (half) h = __shfl_sync(0xffffffffu, h, 0);
+      h *= 0.5 * t;
+      p0 = fma(-h, x0, p0);
+      p1 = fma(-h, x1, p1);
+      if (lane < s) ws[lane] = p0;
+      if (wide && l1 < s) ws[l1] = p1;
+      __syncwarp();
+#pragma unroll 2
+      for (int r = j + 1 + warp; r < s; r += nw) {
+        const double vk = vs[r], wk = ws[r];
+        if (lane > j && lane < s) A[r * ld + lane] -= fma(vk, p0, wk * x0);
+        if (wide && l1 > j && l1 < s) A[r * ld + l1] -= fma(vk, p1, wk * x1);
+      }
+    }
+    if (threadIdx.x == 0) {
+      d[j] = diag;
+      e[j] = beta;
+      tau[j] = t;
+    }
+    hh_barrier(multi);
+    if (warp == 0) {  // v over row j, which no later step reads
+      if (lane > j && lane < s) A[j * ld + lane] = x0;
+      if (wide && l1 > j && l1 < s) A[j * ld + l1] = x1;
+    }
+  }
+  if (threadIdx.x == 0) {
+    d[s - 2] = A[(s - 2) * ld + s - 2];
+    e[s - 2] = A[(s - 2) * ld + s - 1];
+    d[s - 1] = A[(s - 1) * ld + s - 1];
+  }
+}
+
+// Eigenvalues of T below x: sign changes of the leading minors of T - x
+// (d, e2 scaled to a norm of about one; two minors a step are rescaled
+// together before they could underflow).  de[i] = (d_i, e_{i-1}^2), padded
+// with (2, 0), a positive pivot, to a multiple of four: four steps' loads are
+// in flight before their chain of products.
+__device__ __forceinline__ int tri_count_below(const double2* de, int s, double x) {
+  double p0 = 0.0, p1 = 1.0;
+  int cnt = 0;
+  for (int i = 0; i < s; i += 4) {
+    double2 t[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) t[u] = de[i + u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double p2 = fma(t[u].x - x, p1, -t[u].y * p0);
+      cnt += static_cast<int>(static_cast<unsigned>(__double2hiint(p2) ^ __double2hiint(p1)) >> 31);
+      p0 = p1;
+      p1 = p2;
+    }
+    if (fabs(p0) < 0x1p-300 && fabs(p1) < 0x1p-300) {
+      p0 *= 0x1p300;
+      p1 *= 0x1p300;
+    }
+  }
+  return cnt;
+}
+
+__device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, double* theta, double* V,
+                               double* work) {
+  __shared__ double d[kTriMax], e[kTriMax], tau[kTriMax], vs[kTriMax], ws[kTriMax];
+  __shared__ __align__(16) double2 de[kTriMax];
+  __shared__ double th[MAXM], G[MAXM * MAXM], sscale;
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int nw = static_cast<int>(blockDim.x >> 5);
+  const int nt = static_cast<int>(blockDim.x);
+  cta_householder(A, s, ld, d, e, tau, vs, ws, work, s > 16 && nw > 1);
+  __syncthreads();
+  // scale by a power of two (exact) to a Gershgorin bound in [1/2, 1)
+  if (warp == 0) {
+    double b = 0.0;
+    for (int i = lane; i < s; i += 32)
+      b = fmax(b, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < s ? fabs(e[i]) : 0.0));
+    b = warp_max(b);
+    int ex = 0;
+    if (b > 0.0 && isfinite(b)) frexp(b, &ex);
+    const double sc = ldexp(1.0, -ex);
+    __syncwarp();
+    for (int i = lane; i < ((s + 3) & ~3); i += 32) {
+      const double es = (i > 0 && i < s) ? e[i - 1] * sc : 0.0;
+      de[i] = i < s ? make_double2(d[i] * sc, es * es) : make_double2(2.0, 0.0);
+    }
+    __syncwarp();
+    for (int i = lane; i < s; i += 32) {
+      d[i] *= sc;
+      if (i + 1 < s) e[i] *= sc;
+    }
+    if (lane == 0) sscale = ldexp(1.0, ex);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < s; i += nt) {
-    const double d = sm.B[i * ld + i];
-    const bool ok = d > 0.0 && isfinite(d);
-    if (!ok) atomicExch(sflag, 1);
-    dsc[i] = ok ? 1.0 / sqrt(d) : 0.0;
+  // ---- eigenvalues and vectors, one warp each ----
+  double2* Lp = reinterpret_cast<double2*>(work) + warp * 2 * kTriMax;  // per warp: two rows
+  for (int q = warp; q < nsel; q += nw) {
+    const int want = largest ? s - 1 - q : q;
+    double lo = -1.0, hi = 1.0;  // the scaled spectrum lies inside
+    for (int round = 0; round < 13 && hi - lo > 0.5 * DBL_EPSILON; ++round) {
+      const double x = fma(hi - lo, (lane + 1) * (1.0 / 33.0), lo);
+      const unsigned m = __ballot_sync(0xffffffffu, tri_count_below(de, s, x) > want);
+      const int l = m ? __ffs(m) - 1 : 32;
+      const double xl = __shfl_sync(0xffffffffu, x, l & 31), xp = __shfl_sync(0xffffffffu, x, (l + 31) & 31);
+      if (l < 32) hi = xl;
+      if (l > 0) lo = xp;
+    }
+    const double t = 0.5 * (lo + hi);
+    // twisted factorisation: the pivots from the top (lane 0) and from the
+    // bottom (lane 1) as ratios of successive minors, whose recurrences need
+    // no division; out[i] = (minor before i, minor at i) in one scale
+    const double tiny = 0.0625 * DBL_EPSILON * DBL_EPSILON;
+    __syncwarp();
+    if (lane < 2) {
+      double2* out = Lp + lane * kTriMax;
+      double p0 = 0.0, p1 = 1.0;
+      for (int c = 0; c < s; ++c) {
+        const int i = lane == 0 ? c : s - 1 - c;
+        const double ee = lane == 0 ? de[i].y : (c > 0 ? de[i + 1].y : 0.0);
+        const double p2 = fma(de[i].x - t, p1, -ee * p0);
+        out[i] = make_double2(p1, p2);
+        p0 = p1;
+        p1 = p2;
+        if ((c & 3) == 3 && fabs(p0) < 0x1p-300 && fabs(p1) < 0x1p-300) {
+          p0 *= 0x1p300;
+          p1 *= 0x1p300;
+        }
+      }
+    }
+    __syncwarp();
+    double gmin = DBL_MAX;
+    int kmin = 0;
+    double lo_r[2], up_r[2];  // z_i = lo z_{i+1} above the twist, z_i = up z_{i-1} below
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int i = lane + 32 * c;
+      lo_r[c] = 0.0;
+      up_r[c] = 0.0;
+      if (i < s) {
+        const double2 f = Lp[i], g = Lp[kTriMax + i];
+        double df = f.y / f.x, dg = g.y / g.x;
+        if (!(fabs(df) >= tiny)) df = tiny;
+        if (!(fabs(dg) >= tiny)) dg = tiny;
+        const double gam = fabs(df + dg - (de[i].x - t));
+        if (gam < gmin) {
+          gmin = gam;
+          kmin = i;
+        }
+        if (i + 1 < s) lo_r[c] = -e[i] / df;
+        if (i > 0) up_r[c] = -e[i - 1] / dg;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double g = __shfl_xor_sync(0xffffffffu, gmin, o);
+      const int k = __shfl_xor_sync(0xffffffffu, kmin, o);
+      if (g < gmin || (g == gmin && k < kmin)) {
+        gmin = g;
+        kmin = k;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if (lane + 32 * c < s) Lp[lane + 32 * c] = make_double2(lo_r[c], up_r[c]);
+    __syncwarp();
+    if (lane < 2) {
+      double z = 1.0;
+      if (lane == 0) {
+        V[kmin * ld + q] = 1.0;
+#pragma unroll 4
+        for (int i = kmin - 1; i >= 0; --i) {
+          z *= Lp[i].x;
+          V[i * ld + q] = z;
+        }
+      } else {
+#pragma unroll 4
+        for (int i = kmin + 1; i < s; ++i) {
+          z *= Lp[i].y;
+          V[i * ld + q] = z;
+        }
+      }
+    }
+    __syncwarp();
+    double n2 = 0.0;
+    for (int i = lane; i < s; i += 32) n2 = fma(V[i * ld + q], V[i * ld + q], n2);
+    n2 = 1.0 / sqrt(warp_sum(n2));
+    for (int i = lane; i < s; i += 32) V[i * ld + q] *= n2;
+    if (lane == 0) th[q] = t;
   }
   __syncthreads();
-  if (*sflag) return false;
-  for (int t = threadIdx.x; t < s * s; t += nt) {
-    const int i = t / s, j = t % s;
-    const double f = dsc[i] * dsc[j];
-    sm.B[i * ld + j] *= f;
-    sm.A[i * ld + j] *= f;
-  }
-  __syncthreads();
-  // ---- Cholesky, one barrier per pivot ----
-  for (int j = 0; j < s; ++j) {
-    const double piv = sm.B[j * ld + j];
-    if (!(piv > chol_tol)) return false;  // the same value in every thread
-    const double inv2 = 1.0 / piv;        // (b_ij / l_jj)(b_kj / l_jj) = b_ij b_kj / b_jj
-    if (threadIdx.x == 0) lsq[j] = sqrt(piv);
-    const int w = s - j - 1;
-    for (int t = threadIdx.x; t < w * w; t += nt) {
-      const int i = j + 1 + t / w, k = j + 1 + t % w;
-      if (k <= i) sm.B[i * ld + k] -= sm.B[i * ld + j] * sm.B[k * ld + j] * inv2;
+  // ---- orthonormalise: V <- V (3/2 I - G/2), quadratic in |G - I| ----
+  bool fine = false;
+  for (int it = 0; it < 4 && !fine; ++it) {
+    int bad = 0, big = 0;
+    for (int t = threadIdx.x; t < nsel * nsel; t += nt) {
+      const int i = t / nsel, j = t - (t / nsel) * nsel;
+      double g = 0.0;
+      for (int k = 0; k < s; ++k) g = fma(V[k * ld + i], V[k * ld + j], g);
+      G[t] = g;
+      const double off = fabs(i == j ? g - 1.0 : g);
+      if (!(off <= 8.0 * DBL_EPSILON)) bad = 1;
+      if (!(off <= 0.05)) big = 1;
+    }
+    if (__syncthreads_or(big)) return false;
+    fine = !__syncthreads_or(bad);
+    if (fine) break;
+    double nv[2];  // s nsel <= 2 x the CTA's threads (s = 3 nsel: 12 x 4, 24 x 8 on 128; 48 x 16 on 512)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int t = threadIdx.x + c * nt;
+      nv[c] = 0.0;
+      if (t < s * nsel) {
+        const int k = t / nsel, i = t - (t / nsel) * nsel;
+        double v = 1.5 * V[k * ld + i];
+        for (int j = 0; j < nsel; ++j) v = fma(-0.5 * V[k * ld + j], G[j * nsel + i], v);
+        nv[c] = v;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int t = threadIdx.x + c * nt;
+      if (t < s * nsel) V[(t / nsel) * ld + t - (t / nsel) * nsel] = nv[c];
     }
     __syncthreads();
   }
-  for (int t = threadIdx.x; t < s * s; t += nt) {  // finish the columns: l_ij = b_ij / sqrt(b_jj)
-    const int i = t / s, j = t % s;
-    if (i > j) sm.B[i * ld + j] /= lsq[j];
-    else if (i == j) sm.B[i * ld + i] = lsq[i];
+  // ---- residual test in the tridiagonal basis ----
+  int off = fine ? 0 : 1;
+  for (int t = threadIdx.x; t < s * nsel; t += nt) {
+    const int i = t / nsel, q = t - (t / nsel) * nsel;
+    double r = (d[i] - th[q]) * V[i * ld + q];
+    if (i > 0) r = fma(e[i - 1], V[(i - 1) * ld + q], r);
+    if (i + 1 < s) r = fma(e[i], V[(i + 1) * ld + q], r);
+    if (!(fabs(r) <= 2e-13)) off = 1;
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < s; i += nt) lsq[i] = 1.0 / lsq[i];
-  __syncthreads();
-  // ---- M = L^-1 (lower), one column per thread, into Z ----
-  for (int c = threadIdx.x; c < s; c += nt) {
-    for (int i = 0; i < c; ++i) sm.Z[i * ld + c] = 0.0;
-    sm.Z[c * ld + c] = lsq[c];
-    for (int i = c + 1; i < s; ++i) {
-      double v = 0.0;
-      for (int k = c; k < i; ++k) v = fma(sm.B[i * ld + k], sm.Z[k * ld + c], v);
-      sm.Z[i * ld + c] = -v * lsq[i];
+  if (__syncthreads_or(off)) return false;
+  // ---- back-transformation, one warp a vector ----
+  for (int q = warp; q < nsel; q += nw) {
+    double z0 = lane < s ? V[lane * ld + q] : 0.0;
+    double z1 = lane + 32 < s ? V[(lane + 32) * ld + q] : 0.0;
+    for (int j = s - 3; j >= 0; --j) {
+      const double v0 = (lane > j && lane < s) ? A[j * ld + lane] : 0.0;
+      const double v1 = (lane + 32 > j && lane + 32 < s) ? A[j * ld + lane + 32] : 0.0;
+      const double c = tau[j] * warp_sum(fma(v0, z0, v1 * z1));
+      z0 = fma(-c, v0, z0);
+      z1 = fma(-c, v1, z1);
     }
+    if (lane < s) V[lane * ld + q] = z0;
+    if (lane + 32 < s) V[(lane + 32) * ld + q] = z1;
+    if (lane == 0) theta[q] = th[q] * sscale;
   }
   __syncthreads();
-  // keep M in B (L is no longer needed)
-  for (int t = threadIdx.x; t < s * s; t += nt) {
-    const int i = t / s, j = t % s;
-    sm.B[i * ld + j] = sm.Z[i * ld + j];
-  }
-  __syncthreads();
-  // ---- C = M A M^T: Y = M A into T, then C = Y M^T into A ----
-  for (int t = threadIdx.x; t < s * s; t += nt) {
-    const int i = t / s, j = t % s;
-    double v = 0.0;
-    for (int k = 0; k <= i; ++k) v = fma(sm.B[i * ld + k], sm.A[k * ld + j], v);
-    sm.T[i * ld + j] = v;
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < s * s; t += nt) {
-    const int i = t / s, j = t % s;
-    if (j < i) continue;  // upper triangle, mirrored below
-    double v = 0.0;
-    for (int k = 0; k <= j; ++k) v = fma(sm.T[i * ld + k], sm.B[j * ld + k], v);
-    double u = 0.0;  // the (j, i) entry, for the symmetrised average
-    for (int k = 0; k <= i; ++k) u = fma(sm.T[j * ld + k], sm.B[i * ld + k], u);
-    const double a = 0.5 * (v + u);
-    sm.A[i * ld + j] = a;
-    sm.A[j * ld + i] = a;
-  }
-  __syncthreads();
-  cta_identity(sm.V, s, ld);
-  __syncthreads();
-  cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red);
-  // ---- selection by ranks (ascending, or descending for `largest`; ties by index) ----
+  return true;
+}
+
+// The generalised Rayleigh-Ritz of cta_rr_general with its serial sections
+// made parallel (rows over warps, columns over lanes: no index division): the
+// D-scale factors one per thread; the elimination of [B | I] in place, one
+// barrier a pivot, which leaves the unit lower L^-1 below the diagonal and the
+// pivots on it, so that M = L^-1 needs no pass of its own; C = M A M^T and the
+// Ritz vectors D M^T V_sel as parallel products; the wanted pairs of C by
+// cta_tri_select.  Same results as cta_rr_general up to rounding.
+__device__ bool cta_rr_general_par(const double* gb, const double* ga, int P, const int* idx, int s, int nsel,
+                                   int largest, double chol_tol, SmallSmem sm, double* dsc, double* theta_out,
+                                   double* red, int* order, int* sflag) {
+  __shared__ double lsq[3 * MAXM];  // 1 / sqrt of the pivots
+  const int ld = sm.ld;
+  const int nt = blockDim.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nt >> 5;
+  int bad = 0;
   for (int i = threadIdx.x; i < s; i += nt) {
-    const double di = sm.A[i * ld + i];
-    int rank = 0;
-    for (int j = 0; j < s; ++j) {
-      const double dj = sm.A[j * ld + j];
-      // ascending and stable; for `largest` the reverse of that order
-      const bool before = largest ? (dj > di || (dj == di && j > i)) : (dj < di || (dj == di && j < i));
-      rank += before ? 1 : 0;
+    const double d = gb[idx[i] * (P + 1)];
+    const bool ok = d > 0.0 && isfinite(d);
+    if (!ok) bad = 1;
+    dsc[i] = ok ? 1.0 / sqrt(d) : 0.0;
+  }
+  if (__syncthreads_or(bad)) return false;
+  for (int i = warp; i < s; i += nw) {
+    const double di = dsc[i];
+    for (int j = lane; j < s; j += 32) {
+      const int src = idx[i] * P + idx[j];
+      const double f = di * dsc[j];
+      sm.B[i * ld + j] = gb[src] * f;
+      sm.A[i * ld + j] = ga[src] * f;
     }
-    order[rank] = i;
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < nsel; q += nt) theta_out[q] = sm.A[order[q] * ld + order[q]];
+  // ---- elimination of [B | I]: column c <= j of row i holds L^-1, the rest B ----
+  for (int j = 0; j < s; ++j) {
+    const double piv = sm.B[j * ld + j];
+    if (!(piv > chol_tol)) return false;  // the same value in every thread
+    const double inv = 1.0 / piv;
+    const double r0 = sm.B[j * ld + min(lane, s - 1)];
+    const double r1 = s > 32 ? sm.B[j * ld + min(lane + 32, s - 1)] : 0.0;
+    for (int i = j + 1 + warp; i < s; i += nw) {
+      double* row = sm.B + i * ld;
+      const double f = row[j] * inv;
+      __syncwarp();
+      if (lane < s) row[lane] = lane == j ? -f : fma(-f, r0, row[lane]);
+      if (lane + 32 < s) row[lane + 32] = lane + 32 == j ? -f : fma(-f, r1, row[lane + 32]);
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < s; i += nt) lsq[i] = 1.0 / sqrt(sm.B[i * ld + i]);
+  __syncthreads();
+  for (int i = warp; i < s; i += nw) {  // M = diag(1 / l_ii) (unit lower inverse)
+    const double f = lsq[i];
+    for (int j = lane; j < s; j += 32) sm.B[i * ld + j] = j < i ? sm.B[i * ld + j] * f : (j == i ? f : 0.0);
+  }
+  __syncthreads();
+  // ---- C = M A M^T: Y = M A, kept transposed in Z with row r rotated by r
+  // (both the transposed store and the row reads are free of bank conflicts),
+  // then C = M Y^T, to A and to T (the copy that the direct route destroys) ----
+  for (int i0 = warp; i0 < s; i0 += 3 * nw) {
+    const int i1 = min(i0 + nw, s - 1), i2 = min(i0 + 2 * nw, s - 1);
+    const double *m0 = sm.B + i0 * ld, *m1 = sm.B + i1 * ld, *m2 = sm.B + i2 * ld;
+    for (int c = lane; c < s; c += 32) {
+      double v0 = 0.0, v1 = 0.0, v2 = 0.0;
+#pragma unroll 4
+      for (int k = 0; k <= i2; ++k) {
+        const double a = sm.A[k * ld + c];
+        v0 = fma(m0[k], a, v0);
+        v1 = fma(m1[k], a, v1);
+        v2 = fma(m2[k], a, v2);
+      }
+      double* z = sm.Z + c * ld;
+      z[i0 + c < s ? i0 + c : i0 + c - s] = v0;
+      if (i0 + nw < s) z[i1 + c < s ? i1 + c : i1 + c - s] = v1;
+      if (i0 + 2 * nw < s) z[i2 + c < s ? i2 + c : i2 + c - s] = v2;
+    }
+  }
+  __syncthreads();
+  for (int i0 = warp; i0 < s; i0 += 3 * nw) {
+    const int i1 = min(i0 + nw, s - 1), i2 = min(i0 + 2 * nw, s - 1);
+    const double *m0 = sm.B + i0 * ld, *m1 = sm.B + i1 * ld, *m2 = sm.B + i2 * ld;
+    for (int c = lane; c < s; c += 32) {
+      double v0 = 0.0, v1 = 0.0, v2 = 0.0;
+#pragma unroll 4
+      for (int k = 0; k <= i2; ++k) {
+        const double y = sm.Z[k * ld + (c + k < s ? c + k : c + k - s)];
+        v0 = fma(m0[k], y, v0);
+        v1 = fma(m1[k], y, v1);
+        v2 = fma(m2[k], y, v2);
+      }
+      sm.A[i0 * ld + c] = v0;
+      sm.T[i0 * ld + c] = v0;
+      if (i0 + nw < s) {
+        sm.A[i1 * ld + c] = v1;
+        sm.T[i1 * ld + c] = v1;
+      }
+      if (i0 + 2 * nw < s) {
+        sm.A[i2 * ld + c] = v2;
+        sm.T[i2 * ld + c] = v2;
+      }
+    }
+  }
+  __syncthreads();
+  // the wanted pairs directly (T: a copy of C to destroy, Z: scratch); Jacobi
+  // on C where that route does not apply or its tests fail (pairs that agree
+  // to rounding)
+  bool direct = false;
+  if (s >= 3 && s * nsel <= 2 * nt) {
+    direct = cta_tri_select(sm.T, s, ld, nsel, largest, theta_out, sm.V, sm.W);
+  }
+  if (direct) {
+    for (int q = threadIdx.x; q < nsel; q += nt) order[q] = q;
+    __syncthreads();
+  } else {
+    cta_identity(sm.V, s, ld);
+    for (int t = threadIdx.x; t < s * s; t += nt) {  // C to exact symmetry
+      const int i = t / s, j = t - (t / s) * s;
+      if (j > i) sm.T[i * ld + j] = 0.5 * (sm.A[i * ld + j] + sm.A[j * ld + i]);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < s * s; t += nt) {
+      const int i = t / s, j = t - (t / s) * s;
+      if (j > i) {
+        sm.A[i * ld + j] = sm.T[i * ld + j];
+        sm.A[j * ld + i] = sm.T[i * ld + j];
+      }
+    }
+    __syncthreads();
+    cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red);
+    // ---- selection by ranks (ascending, or descending for `largest`; ties by index) ----
+    for (int i = threadIdx.x; i < s; i += nt) {
+      const double di = sm.A[i * ld + i];
+      int rank = 0;
+      for (int j = 0; j < s; ++j) {
+        const double dj = sm.A[j * ld + j];
+        // ascending and stable; for `largest` the reverse of that order
+        const bool before = largest ? (dj > di || (dj == di && j > i)) : (dj < di || (dj == di && j < i));
+        rank += before ? 1 : 0;
+      }
+      order[rank] = i;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < nsel; q += nt) theta_out[q] = sm.A[order[q] * ld + order[q]];
+  }
   // ---- Z = D M^T V_sel ----
   for (int t = threadIdx.x; t < s * nsel; t += nt) {
-    const int i = t / nsel, q = t % nsel;
+    const int i = t / nsel, q = t - (t / nsel) * nsel;
     const int c = order[q];
     double v = 0.0;
+#pragma unroll 4
     for (int k = i; k < s; ++k) v = fma(sm.B[k * ld + i], sm.V[k * ld + c], v);
     sm.Z[i * ld + q] = v * dsc[i];
   }
@@ -921,20 +1320,36 @@ __device__ bool rr_general(const double* gb, const double* ga, int P, const int*
                         sflag);
 }
 
-// `ctrl` points to the CTA's shared-memory copy of the control block.
+// `ctrl` points to the CTA's shared-memory copy of the control block's header;
+// the coefficients, which the step only writes, go to `gctrl` in global memory.
 template <int NT, bool REG, bool PAR>
-__device__ void small_step_body(LobpcgCtrl* ctrl, const double* __restrict__ gram, int ns, int mode,
+__device__ void small_step_body(LobpcgCtrl* ctrl, LobpcgCtrl* gctrl, const double* __restrict__ gram, int ns, int mode,
                                 double* smem) {
   __shared__ double red[ST_WIDE / 32];
   __shared__ double rc[SMAX / 2 + 1], rs[SMAX / 2 + 1], dsc[3 * MAXM], theta[MAXM], rn[MAXM];
-  __shared__ int ra[SMAX / 2 + 1], rb[SMAX / 2 + 1], order[3 * MAXM], idx[3 * MAXM];
+  __shared__ int ra[SMAX / 2 + 1], rb[SMAX / 2 + 1], order[3 * MAXM], idx[3 * MAXM], inv[3 * MAXM];
   __shared__ int sflag, sdone, s_na, s_withp;
   const int LDS = 3 * MAXM;
-  SmallSmem sm{smem, smem + LDS * LDS, smem + 2 * LDS * LDS, smem + 3 * LDS * LDS, smem + 4 * LDS * LDS, LDS};
+  SmallSmem sm{smem, smem + LDS * LDS, smem + 2 * LDS * LDS, smem + 3 * LDS * LDS, smem + 4 * LDS * LDS, LDS,
+               smem + 5 * LDS * LDS};
   const int m = ctrl->m;
   const int P = ns * m;
   const double* gb = gram;
   const double* ga = gram + P * P;
+  if (mode == SM_ITER) {
+    if constexpr (PAR) {
+      // both Gram matrices to shared memory in one go, in flight with the
+      // residual norms below (V and T are free until the eigensolve)
+      for (int t = threadIdx.x; t < P * P; t += blockDim.x) {
+        sm.V[t] = gb[t];
+        sm.T[t] = ga[t];
+      }
+    }
+    for (int c = threadIdx.x; c < m; c += blockDim.x) {
+      const double g = gb[(m + c) * P + (m + c)];
+      rn[c] = sqrt(g > 0.0 ? g : 0.0);
+    }
+  }
   if (threadIdx.x == 0) {
     sdone = ctrl->done;
     // iterations queued after convergence: the final best copy already happened
@@ -968,9 +1383,9 @@ __device__ void small_step_body(LobpcgCtrl* ctrl, const double* __restrict__ gra
     if (ok) {
       for (int t = threadIdx.x; t < MAXM * MAXM; t += blockDim.x) {
         const int i = t / MAXM, q = t % MAXM;
-        ctrl->Cx[t] = (i < m && q < m) ? sm.Z[i * LDS + q] : 0.0;
-        ctrl->Cr[t] = 0.0;
-        ctrl->Cp[t] = 0.0;
+        gctrl->Cx[t] = (i < m && q < m) ? sm.Z[i * LDS + q] : 0.0;
+        gctrl->Cr[t] = 0.0;
+        gctrl->Cp[t] = 0.0;
       }
     }
     return;
@@ -989,7 +1404,7 @@ __device__ void small_step_body(LobpcgCtrl* ctrl, const double* __restrict__ gra
     __syncthreads();
     for (int t = threadIdx.x; t < MAXM * MAXM; t += blockDim.x) {
       const int i = t / MAXM, q = t % MAXM;
-      ctrl->Cx[t] = (i < m && q < m) ? sm.V[i * LDS + order[q]] : 0.0;
+      gctrl->Cx[t] = (i < m && q < m) ? sm.V[i * LDS + order[q]] : 0.0;
     }
     return;
   }
@@ -1005,59 +1420,55 @@ __device__ void small_step_body(LobpcgCtrl* ctrl, const double* __restrict__ gra
     }
     for (int t = threadIdx.x; t < MAXM * MAXM; t += blockDim.x) {
       const int i = t / MAXM, q = t % MAXM;
-      ctrl->Cx[t] = (ok && i < m && q < m) ? sm.Z[i * LDS + q] : 0.0;
+      gctrl->Cx[t] = (ok && i < m && q < m) ? sm.Z[i * LDS + q] : 0.0;
     }
     if (threadIdx.x == 0) ctrl->status = ok ? ST_CONVERGED : ST_BREAKDOWN;
     return;
   }
 
   // ---- SM_ITER --------------------------------------------------------------
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {  // warp 0, lane c = column c
     const int k = ctrl->k_wanted;
+    const int c = threadIdx.x;
+    const bool mine = c < m;
     double sum = 0.0;
-    for (int c = 0; c < m; ++c) {
-      const double g = gb[(m + c) * P + (m + c)];
-      rn[c] = sqrt(g > 0.0 ? g : 0.0);
+    for (int j = 0; j < k; ++j) sum += rn[j];
+    const bool copy = ctrl->best_sum > sum;
+    const bool capped = ctrl->iter >= ctrl->maxiter;
+    const int act = mine && (c >= k || (ctrl->active[c] && rn[c] > ctrl->tol)) ? 1 : 0;
+    const unsigned am = __ballot_sync(0xffffffffu, act);
+    const unsigned wanted = k < 32 ? (1u << k) - 1u : 0xffffffffu;
+    const bool conv = (am & wanted) == 0u;
+    if (mine) {
       ctrl->rnorm[c] = rn[c];
-      if (c < k) sum += rn[c];
-    }
-    int copy = 0;
-    if (ctrl->best_sum > sum) {
-      ctrl->best_sum = sum;
-      ctrl->best_iter = ctrl->iter;
-      for (int c = 0; c < m; ++c) {
+      ctrl->active[c] = act;
+      if (copy) {
         ctrl->best_lam[c] = ctrl->lam[c];
         ctrl->best_rnorm[c] = rn[c];
       }
-      copy = 1;
-    }
-    ctrl->copy_best = copy;
-    int na_wanted = 0;
-    for (int c = 0; c < m; ++c) {
-      if (c < k) {
-        ctrl->active[c] = (ctrl->active[c] && rn[c] > ctrl->tol) ? 1 : 0;
-        na_wanted += ctrl->active[c];
-      } else {
-        ctrl->active[c] = 1;
+      idx[c] = c;
+      if (act) {
+        const int at = m + __popc(am & ((1u << c) - 1u));
+        idx[at] = m + c;                  // R, then P, of the active columns
+        idx[at + __popc(am)] = 2 * m + c;
       }
     }
-    int done = 0;
-    if (na_wanted == 0) {
-      done = 1;
-      ctrl->status = ST_CONVERGED;
-    } else if (ctrl->iter >= ctrl->maxiter) {
-      done = 1;
-      ctrl->status = ST_MAXITER;
+    __syncwarp();
+    if (c == 0) {
+      if (copy) {
+        ctrl->best_sum = sum;
+        ctrl->best_iter = ctrl->iter;
+      }
+      ctrl->copy_best = copy ? 1 : 0;
+      if (conv) ctrl->status = ST_CONVERGED;
+      else if (capped) ctrl->status = ST_MAXITER;
+      const int done = conv || capped ? 1 : 0;
+      ctrl->done = done;
+      sdone = done;
+      if (!done) ctrl->iter += 1;
+      s_na = __popc(am);
+      s_withp = ctrl->p_valid;
     }
-    ctrl->done = done;
-    sdone = done;
-    if (!done) ctrl->iter += 1;
-    int na = 0;
-    for (int c = 0; c < m; ++c)
-      if (ctrl->active[c]) idx[m + na++] = m + c;
-    for (int c = 0; c < m; ++c) idx[c] = c;
-    s_na = na;
-    s_withp = ctrl->p_valid;
   }
   __syncthreads();
   if (sdone) return;
@@ -1065,14 +1476,8 @@ __device__ void small_step_body(LobpcgCtrl* ctrl, const double* __restrict__ gra
   bool ok = false;
   int withp = s_withp;
   if (withp) {
-    if (threadIdx.x == 0) {
-      int q = 0;
-      for (int c = 0; c < m; ++c)
-        if (ctrl->active[c]) idx[m + na + q++] = 2 * m + c;
-    }
-    __syncthreads();
-    ok = rr_general<NT, REG, PAR>(gb, ga, P, idx, m + 2 * na, m, ctrl->largest, ctrl->chol_tol, sm, dsc, theta, red, rc, rs,
-                        ra, rb, order, &sflag);
+    ok = rr_general<NT, REG, PAR>(PAR ? sm.V : gb, PAR ? sm.T : ga, P, idx, m + 2 * na, m, ctrl->largest,
+                                  ctrl->chol_tol, sm, dsc, theta, red, rc, rs, ra, rb, order, &sflag);
     if (!ok) withp = 0;
   }
   if (!ok) {
@@ -1086,23 +1491,19 @@ __device__ void small_step_body(LobpcgCtrl* ctrl, const double* __restrict__ gra
     }
     return;
   }
-  // scatter the coefficients
-  for (int t = threadIdx.x; t < MAXM * MAXM; t += blockDim.x) {
-    ctrl->Cx[t] = 0.0;
-    ctrl->Cr[t] = 0.0;
-    ctrl->Cp[t] = 0.0;
-  }
+  // the coefficients of X, R, P from the rows of Z (zero for what the step left
+  // out; the entries outside m x m were zeroed by the initial step)
+  const int rows = m + na * (withp ? 2 : 1);
+  for (int t = threadIdx.x; t < 3 * MAXM; t += blockDim.x) inv[t] = -1;
   __syncthreads();
-  for (int t = threadIdx.x; t < (m + na * (withp ? 2 : 1)) * m; t += blockDim.x) {
-    const int row = t / m, q = t % m;
-    const double v = sm.Z[row * LDS + q];
-    const int col = idx[row];
-    if (col < m)
-      ctrl->Cx[col * MAXM + q] = v;
-    else if (col < 2 * m)
-      ctrl->Cr[(col - m) * MAXM + q] = v;
-    else
-      ctrl->Cp[(col - 2 * m) * MAXM + q] = v;
+  for (int t = threadIdx.x; t < rows; t += blockDim.x) inv[idx[t]] = t;
+  __syncthreads();
+  for (int t = threadIdx.x; t < 3 * m * MAXM; t += blockDim.x) {
+    const int c = t / MAXM, q = t % MAXM;
+    const int blk = c < m ? 0 : (c < 2 * m ? 1 : 2);
+    const int row = inv[c];
+    double* dst = blk == 0 ? gctrl->Cx : (blk == 1 ? gctrl->Cr : gctrl->Cp);
+    if (q < m) dst[(c - blk * m) * MAXM + q] = row >= 0 ? sm.Z[row * LDS + q] : 0.0;
   }
   if (threadIdx.x == 0) {
     for (int q = 0; q < m; ++q) ctrl->lam[q] = theta[q];
@@ -1111,20 +1512,21 @@ __device__ void small_step_body(LobpcgCtrl* ctrl, const double* __restrict__ gra
   }
 }
 
-// The control block is staged in shared memory for the whole step (the step
-// is a long chain of small dependent updates) and written back at the end.
+// The control block's header is staged in shared memory for the whole step
+// (the step is a long chain of small dependent updates) and written back at
+// the end.
 template <int NT, bool REG = false, bool PAR = false>
 __global__ void __launch_bounds__(NT, 1) k_small_step(LobpcgCtrl* ctrl, const double* __restrict__ gram, int ns,
                                                    int mode) {
   extern __shared__ double smem[];
   __shared__ LobpcgCtrl sctrl;
-  static_assert(sizeof(LobpcgCtrl) % sizeof(double) == 0, "control block must be a whole number of words");
-  constexpr int W = sizeof(LobpcgCtrl) / sizeof(double);
+  constexpr int W = offsetof(LobpcgCtrl, Cx) / sizeof(double);
+  static_assert(offsetof(LobpcgCtrl, Cx) % sizeof(double) == 0, "the header must be a whole number of words");
   double* dst = reinterpret_cast<double*>(&sctrl);
   const double* src = reinterpret_cast<const double*>(ctrl);
   for (int i = threadIdx.x; i < W; i += blockDim.x) dst[i] = src[i];
   __syncthreads();
-  small_step_body<NT, REG, PAR>(&sctrl, gram, ns, mode, smem);
+  small_step_body<NT, REG, PAR>(&sctrl, ctrl, gram, ns, mode, smem);
   __syncthreads();
   double* back = reinterpret_cast<double*>(ctrl);
   for (int i = threadIdx.x; i < W; i += blockDim.x) back[i] = dst[i];
@@ -1186,7 +1588,7 @@ int small_step_variant() {
 
 void small_step_dev(const Exec& ex, LobpcgCtrl* ctrl, const double* gram, int ns, int mode, int m) {
   const int LDS = 3 * MAXM;
-  const size_t smem = sizeof(double) * 5 * LDS * LDS;
+  const size_t smem = sizeof(double) * (5 * LDS * LDS + kTriWork);
   static std::atomic<bool> attr_set[128];
   if (ex.device >= 0 && ex.device < 128 && !attr_set[ex.device]) {
     SI_CUDA(cudaFuncSetAttribute(k_small_step<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
