@@ -804,122 +804,219 @@ constexpr int kTriMax = 3 * MAXM;
 constexpr int kTriWarps = 16;  // warps that take an eigenpair each
 constexpr int kTriWork = kTriWarps * 4 * kTriMax;  // doubles of scratch
 
-// Householder tridiagonalisation.  Lane l owns columns l and l + 32; the rows
-// of the symmetric matrix are split over the engaged warps (one, without
-// barriers, up to 16 columns; four above, where more warps only re-read the
-// partial products: 16 warps cost 3.3 k cycles a column at 48 x 48).  Every
-// engaged warp forms the reflector and w redundantly, so a column costs two
-// barriers.  H = I - tau v v^T with v_{j+1} = alpha - beta unnormalised: the
-// one division, tau = 1 / (beta (beta - alpha)), overlaps the product A v.
-__device__ __forceinline__ void hh_barrier(bool multi) {
-  if (multi) asm volatile("bar.sync 1, 128;" ::: "memory");
-  else __syncwarp();
+// Householder tridiagonalisation, the matrix in registers throughout.
+// H_j = I - tau v v^T with v = (alpha - beta, x_{j+2}, ...) unnormalised: its
+// division, tau = 1 / (beta (beta - alpha)), overlaps the product A v.  Row j
+// of A receives v, d / e / tau the tridiagonal and the factors.
+struct Reflector {
+  double beta, v1, tau_inv;  // v1: v's first element; tau_inv = 0: H = I
+};
+__device__ __forceinline__ Reflector make_reflector(double alpha, double sigma) {
+  Reflector r{alpha, 0.0, 0.0};
+  if (sigma > 0.0) {
+    const double nrm = sqrt(fma(alpha, alpha, sigma));
+    r.beta = alpha >= 0.0 ? -nrm : nrm;
+    r.v1 = alpha - r.beta;
+    r.tau_inv = -r.beta * r.v1;
+  }
+  return r;
 }
 
-__device__ __forceinline__ double warp_sum_low(double v, bool half) {
-  // lanes 16..31 hold zero when half: one level less
-  if (!half) v += __shfl_xor_sync(0xffffffffu, v, 16);
+// Up to N <= 32 columns in one warp: lane l holds column l, a[k] = A(j + k, l)
+// with the rows moved up by one register per column, so that every index is
+// static while the column loop stays a loop.  A column costs two round trips
+// through shared memory (row j, then p = A v, each read by every lane, which
+// then forms the sums, v and w itself) and no shuffle: 0.55 k cycles at 12 x
+// 12 against 1.7 k with the matrix in shared memory and shuffle reductions.
+template <int N>
+__device__ void warp_householder(double* A, int s, int ld, double* d, double* e, double* tau, double* xs, double* ps) {
+  const int l = threadIdx.x & 31;
+  double a[N];
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int k = 0; k < N; ++k) a[k] = (k < s && l < s) ? A[k * ld + l] : 0.0;
+  __syncwarp();
+#pragma unroll 1
+  for (int j = 0; j + 2 < s; ++j) {
+    const int at = l >= j ? l - j : l - j + N;  // slot 0: the diagonal, 1: alpha, 2 ..: below; zero past the end
+    if (l < N) xs[at] = l >= j ? a[0] : 0.0;
+    __syncwarp();
+    double v[N];
+#pragma unroll
+    for (int k = 0; k < N; k += 2) {
+      const double2 t = *reinterpret_cast<const double2*>(xs + k);
+      v[k] = t.x;
+      v[k + 1] = t.y;
+    }
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int k = 2; k < N; k += 2) {
+      s0 = fma(v[k], v[k], s0);
+      s1 = fma(v[k + 1], v[k + 1], s1);
+    }
+    const Reflector r = make_reflector(v[1], s0 + s1);
+    const double diag = v[0];
+    const bool on = r.tau_inv != 0.0;
+    const double own = l == j + 1 ? r.v1 : (l > j ? a[0] : 0.0);
+    const double tj = on ? 1.0 / r.tau_inv : 0.0;
+    v[1] = r.v1;
+    s0 = 0.0;
+    s1 = 0.0;
+#pragma unroll
+    for (int k = 1; k + 1 < N; k += 2) {
+      s0 = fma(a[k], v[k], s0);
+      s1 = fma(a[k + 1], v[k + 1], s1);
+    }
+    s0 = fma(a[N - 1], v[N - 1], s0);
+    const double p = l > j ? s0 + s1 : 0.0;
+    if (l < N) ps[at] = p;
+    __syncwarp();
+    double w[N];
+#pragma unroll
+    for (int k = 0; k < N; k += 2) {
+      const double2 t = *reinterpret_cast<const double2*>(ps + k);
+      w[k] = t.x;
+      w[k + 1] = t.y;
+    }
+    s0 = 0.0;
+    s1 = 0.0;
+#pragma unroll
+    for (int k = 1; k + 1 < N; k += 2) {
+      s0 = fma(w[k], v[k], s0);
+      s1 = fma(w[k + 1], v[k + 1], s1);
+    }
+    s0 = fma(w[N - 1], v[N - 1], s0);
+    const double h = 0.5 * tj * tj * (s0 + s1);  // w = tau p - h v
+    const double wown = fma(tj, p, -h * own);
+#pragma unroll
+    for (int k = 1; k < N; ++k) {
+      w[k] = fma(tj, w[k], -h * v[k]);
+      a[k - 1] = on ? a[k] - fma(v[k], wown, w[k] * own) : a[k];
+    }
+    a[N - 1] = 0.0;
+    if (l > j && l < s) A[j * ld + l] = on ? own : 0.0;
+    if (l == 0) {
+      d[j] = diag;
+      e[j] = r.beta;
+      tau[j] = tj;
+    }
+    __syncwarp();
+  }
+  // the last two rows: a[0], a[1] of lanes s - 2, s - 1
+  if (l == s - 2) d[s - 2] = a[0];
+  if (l == s - 1) {
+    e[s - 2] = a[0];
+    d[s - 1] = a[1];
+  }
 }
 
-__device__ void cta_householder(double* A, int s, int ld, double* d, double* e, double* tau, double* vs, double* ws,
-                                double* part, bool multi) {
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int nw = multi ? 4 : 1;
-  if (warp >= nw) return;
+// Sum over the warp of four values at once: every level halves the values a
+// lane carries, 6 shuffles (of doubles) for all four instead of 20.  On return
+// lane l holds the sum of value ((l >> 4) & 1) * 2 + ((l >> 3) & 1).
+__device__ __forceinline__ double warp_sum4(double v0, double v1, double v2, double v3, int lane) {
+  const bool h = lane & 16;
+  double k0 = (h ? v2 : v0) + __shfl_xor_sync(0xffffffffu, h ? v0 : v2, 16);
+  const double k1 = (h ? v3 : v1) + __shfl_xor_sync(0xffffffffu, h ? v1 : v3, 16);
+  const bool g = lane & 8;
+  k0 = (g ? k1 : k0) + __shfl_xor_sync(0xffffffffu, g ? k0 : k1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) k0 += __shfl_xor_sync(0xffffffffu, k0, o);
+  return k0;
+}
+
+// Up to 48 columns over 16 warps: warp w holds rows w, w + 16, w + 32, lane l
+// columns l and l + 32.  The warp that owns the next row forms its reflector
+// and publishes it; p = A v is a row sum, v^T p a sum of one partial per warp:
+// two barriers a column and few shuffles, which bound this kernel (one a cycle
+// for the SM: every warp summing for itself cost 2.1 k cycles a column).
+__device__ void cta_householder48(double* A, int s, int ld, double* d, double* e, double* tau, double* xs, double* ps) {
+  constexpr int NW = ST_WIDE / 32;
+  static_assert(3 * NW == kTriMax, "three rows a warp");
+  __shared__ __align__(16) double part[NW];
+  __shared__ Reflector refl;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int l1 = lane + 32;
-  const bool wide = s > 32;
-  const bool half = s <= 16;
+  double a0[3], a1[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int r = warp + q * NW;
+    a0[q] = (r < s && lane < s) ? A[r * ld + lane] : 0.0;
+    a1[q] = (r < s && l1 < s) ? A[r * ld + l1] : 0.0;
+  }
+  // row r (x0, x1 on its lanes), its reflector and its diagonal entry
+  auto publish = [&](int r, double x0, double x1) {
+    double sq = lane > r + 1 ? x0 * x0 : 0.0;
+    if (l1 > r + 1) sq = fma(x1, x1, sq);
+    const double sigma = warp_sum(sq);
+    const double alpha = __shfl_sync(0xffffffffu, r + 1 < 32 ? x0 : x1, (r + 1) & 31);
+    const double diag = __shfl_sync(0xffffffffu, r < 32 ? x0 : x1, r & 31);
+    const Reflector f = make_reflector(alpha, sigma);
+    const bool on = f.tau_inv != 0.0;
+    x0 = lane == r + 1 ? f.v1 : (on && lane > r ? x0 : 0.0);
+    x1 = l1 == r + 1 ? f.v1 : (on && l1 > r ? x1 : 0.0);
+    xs[lane] = x0;
+    if (l1 < kTriMax) xs[l1] = x1;
+    if (lane > r && lane < s) A[r * ld + lane] = x0;
+    if (l1 > r && l1 < s) A[r * ld + l1] = x1;
+    if (lane == 0) {
+      refl = f;
+      d[r] = diag;
+      e[r] = f.beta;
+    }
+  };
+  if (warp == 0) publish(0, a0[0], a1[0]);
+  __syncthreads();
+#pragma unroll 1
   for (int j = 0; j + 2 < s; ++j) {
-    const double* row = A + j * ld;
-    double x0 = (lane > j && lane < s) ? row[lane] : 0.0;
-    double x1 = (wide && l1 > j && l1 < s) ? row[l1] : 0.0;
-    const double alpha = row[j + 1];
-    const double diag = row[j];
-    double sq = lane == j + 1 ? 0.0 : x0 * x0;
-    if (l1 != j + 1) sq = fma(x1, x1, sq);
-    // half: the sum is over lanes 0..15 and read back from lane 0's half
-    double sigma = warp_sum_low(sq, half);
-    if (half) sigma = __shfl_sync(0xffffffffu, sigma, 0);
-    double t = 0.0, beta = alpha;
-    if (sigma > 0.0) {
-      const double nrm = sqrt(fma(alpha, alpha, sigma));
-      beta = alpha >= 0.0 ? -nrm : nrm;
-      t = beta * (beta - alpha);  // its reciprocal below
-      if (lane == j + 1) x0 = alpha - beta;
-      if (l1 == j + 1) x1 = alpha - beta;
-    } else {
-      x0 = 0.0;
-      x1 = 0.0;
+    const double x0 = xs[lane], x1 = l1 < kTriMax ? xs[l1] : 0.0;
+    const double ti = refl.tau_inv;
+    const double tj = ti != 0.0 ? 1.0 / ti : 0.0;
+    double vr[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) vr[q] = xs[warp + q * NW];
+    const double sum = warp_sum4(fma(a0[0], x0, a1[0] * x1), fma(a0[1], x0, a1[1] * x1), fma(a0[2], x0, a1[2] * x1),
+                                 0.0, lane);
+    double p[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) p[q] = __shfl_sync(0xffffffffu, sum, q * 8);
+    if (lane == 0) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) ps[warp + q * NW] = p[q];
+      part[warp] = fma(p[0], vr[0], fma(p[1], vr[1], p[2] * vr[2]));  // v is zero at rows <= j
     }
-    // the same values from every engaged warp; rewritten only after the barrier that ends the column
-    if (lane < s) vs[lane] = x0;
-    if (wide && l1 < s) vs[l1] = x1;
-    __syncwarp();
-    if (t != 0.0) {
-      t = 1.0 / t;
-      double p0 = 0.0, p1 = 0.0, r0 = 0.0, r1 = 0.0;
-      int k = j + 1 + warp;
-      const int c0 = min(lane, s - 1), c1 = wide ? min(l1, s - 1) : 0;
-      for (; k + nw < s; k += 2 * nw) {
-        const double va = vs[k], vb = vs[k + nw];
-        p0 = fma(A[k * ld + c0], va, p0);
-        r0 = fma(A[(k + nw) * ld + c0], vb, r0);
-        if (wide) {
-          p1 = fma(A[k * ld + c1], va, p1);
-          r1 = fma(A[(k + nw) * ld + c1], vb, r1);
-        }
-      }
-      if (k < s) {
-        p0 = fma(A[k * ld + c0], vs[k], p0);
-        if (wide) p1 = fma(A[k * ld + c1], vs[k], p1);
-      }
-      p0 += r0;
-      p1 += r1;
-      if (multi) {
-        part[warp * kTriMax + lane] = p0;
-        if (l1 < kTriMax) part[warp * kTriMax + l1] = p1;
-        hh_barrier(true);
-        p0 = (part[lane] + part[kTriMax + lane]) + (part[2 * kTriMax + lane] + part[3 * kTriMax + lane]);
-        if (l1 < kTriMax)
-          p1 = (part[l1] + part[kTriMax + l1]) + (part[2 * kTriMax + l1] + part[3 * kTriMax + l1]);
-      }
-      p0 *= t;
-      p1 *= t;
-      // x is zero outside columns j + 1 .. s - 1
-      double h = warp_sum_low(fma(p0, x0, p1 * x1), half);
-      if (half) h = __shfl_sync(0xffffffffu, h, 0);
-      h *= 0.5 * t;
-      p0 = fma(-h, x0, p0);
-      p1 = fma(-h, x1, p1);
-      if (lane < s) ws[lane] = p0;
-      if (wide && l1 < s) ws[l1] = p1;
-      __syncwarp();
-#pragma unroll 2
-      for (int r = j + 1 + warp; r < s; r += nw) {
-        const double vk = vs[r], wk = ws[r];
-        if (lane > j && lane < s) A[r * ld + lane] -= fma(vk, p0, wk * x0);
-        if (wide && l1 > j && l1 < s) A[r * ld + l1] -= fma(vk, p1, wk * x1);
-      }
+    __syncthreads();
+    const double q0 = ps[lane], q1 = l1 < kTriMax ? ps[l1] : 0.0;
+    double h0 = 0.0, h1 = 0.0;
+#pragma unroll
+    for (int w = 0; w < NW; w += 2) {
+      const double2 t = *reinterpret_cast<const double2*>(part + w);
+      h0 += t.x;
+      h1 += t.y;
     }
-    if (threadIdx.x == 0) {
-      d[j] = diag;
-      e[j] = beta;
-      tau[j] = t;
+    const double h = 0.5 * tj * tj * (h0 + h1);  // w = tau p - h v
+    // rows and columns <= j keep whatever they hold: nothing reads them again
+    const double w0 = fma(tj, q0, -h * x0), w1 = fma(tj, q1, -h * x1);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double wr = fma(tj, p[q], -h * vr[q]);
+      a0[q] -= fma(vr[q], w0, wr * x0);
+      a1[q] -= fma(vr[q], w1, wr * x1);
     }
-    hh_barrier(multi);
-    if (warp == 0) {  // v over row j, which no later step reads
-      if (lane > j && lane < s) A[j * ld + lane] = x0;
-      if (wide && l1 > j && l1 < s) A[j * ld + l1] = x1;
+    if (threadIdx.x == 0) tau[j] = tj;
+    if (j + 3 < s) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (warp + q * NW == j + 1) publish(j + 1, a0[q], a1[q]);
+      __syncthreads();
     }
   }
-  if (threadIdx.x == 0) {
-    d[s - 2] = A[(s - 2) * ld + s - 2];
-    e[s - 2] = A[(s - 2) * ld + s - 1];
-    d[s - 1] = A[(s - 1) * ld + s - 1];
+  // the last two rows from their owners
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int r = warp + q * NW;
+    if (r == s - 2 || r == s - 1) {
+      if (lane == (r & 31)) d[r] = r < 32 ? a0[q] : a1[q];
+      if (r == s - 2 && lane == ((s - 1) & 31)) e[r] = s - 1 < 32 ? a0[q] : a1[q];
+    }
   }
 }
 
@@ -930,6 +1027,7 @@ __device__ void cta_householder(double* A, int s, int ld, double* d, double* e, 
 // in flight before their chain of products.
 __device__ __forceinline__ int tri_count_below(const double2* de, int s, double x) {
   double p0 = 0.0, p1 = 1.0;
+  unsigned signs = 0;  // one bit a step, the previous step's sign in the bit above
   int cnt = 0;
   for (int i = 0; i < s; i += 4) {
     double2 t[4];
@@ -938,10 +1036,11 @@ __device__ __forceinline__ int tri_count_below(const double2* de, int s, double 
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const double p2 = fma(t[u].x - x, p1, -t[u].y * p0);
-      cnt += static_cast<int>(static_cast<unsigned>(__double2hiint(p2) ^ __double2hiint(p1)) >> 31);
+      signs = __funnelshift_l(static_cast<unsigned>(__double2hiint(p2)), signs, 1);
       p0 = p1;
       p1 = p2;
     }
+    cnt += __popc((signs ^ (signs >> 1)) & 15u);
     if (fabs(p0) < 0x1p-300 && fabs(p1) < 0x1p-300) {
       p0 *= 0x1p300;
       p1 *= 0x1p300;
@@ -952,14 +1051,17 @@ __device__ __forceinline__ int tri_count_below(const double2* de, int s, double 
 
 __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, double* theta, double* V,
                                double* work) {
-  __shared__ double d[kTriMax], e[kTriMax], tau[kTriMax], vs[kTriMax], ws[kTriMax];
+  __shared__ double d[kTriMax], e[kTriMax], tau[kTriMax];
+  __shared__ __align__(16) double vs[kTriMax], ws[kTriMax];
   __shared__ __align__(16) double2 de[kTriMax];
   __shared__ double th[MAXM], G[MAXM * MAXM], sscale;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int nw = static_cast<int>(blockDim.x >> 5);
   const int nt = static_cast<int>(blockDim.x);
-  cta_householder(A, s, ld, d, e, tau, vs, ws, work, s > 16 && nw > 1);
+  if (nt == ST_WIDE) cta_householder48(A, s, ld, d, e, tau, vs, ws);
+  else if (warp == 0 && s <= 16) warp_householder<16>(A, s, ld, d, e, tau, vs, ws);
+  else if (warp == 0) warp_householder<24>(A, s, ld, d, e, tau, vs, ws);
   __syncthreads();
   // scale by a power of two (exact) to a Gershgorin bound in [1/2, 1)
   if (warp == 0) {
@@ -967,9 +1069,11 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
     for (int i = lane; i < s; i += 32)
       b = fmax(b, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < s ? fabs(e[i]) : 0.0));
     b = warp_max(b);
-    int ex = 0;
-    if (b > 0.0 && isfinite(b)) frexp(b, &ex);
-    const double sc = ldexp(1.0, -ex);
+    // exponent field of b, kept where 2^-ex is a normal number (a bound outside
+    // that range, or none, leaves T unscaled: the tests below then decide)
+    const int be = (__double2hiint(b) >> 20) & 0x7ff;
+    const int ex = be > 32 && be < 2014 ? be - 1022 : 0;
+    const double sc = __hiloint2double((1023 - ex) << 20, 0);
     __syncwarp();
     for (int i = lane; i < ((s + 3) & ~3); i += 32) {
       const double es = (i > 0 && i < s) ? e[i - 1] * sc : 0.0;
@@ -980,7 +1084,7 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
       d[i] *= sc;
       if (i + 1 < s) e[i] *= sc;
     }
-    if (lane == 0) sscale = ldexp(1.0, ex);
+    if (lane == 0) sscale = __hiloint2double((1023 + ex) << 20, 0);
   }
   __syncthreads();
   // ---- eigenvalues and vectors, one warp each ----
@@ -1005,14 +1109,22 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
     if (lane < 2) {
       double2* out = Lp + lane * kTriMax;
       double p0 = 0.0, p1 = 1.0;
-      for (int c = 0; c < s; ++c) {
-        const int i = lane == 0 ? c : s - 1 - c;
-        const double ee = lane == 0 ? de[i].y : (c > 0 ? de[i + 1].y : 0.0);
-        const double p2 = fma(de[i].x - t, p1, -ee * p0);
-        out[i] = make_double2(p1, p2);
-        p0 = p1;
-        p1 = p2;
-        if ((c & 3) == 3 && fabs(p0) < 0x1p-300 && fabs(p1) < 0x1p-300) {
+      for (int c0 = 0; c0 < s; c0 += 4) {
+        double dd[4], ee[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = min(c0 + u, s - 1);
+          dd[u] = de[lane == 0 ? c : s - 1 - c].x - t;
+          ee[u] = lane == 0 ? de[c].y : (c > 0 ? de[s - c].y : 0.0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double p2 = fma(dd[u], p1, -ee[u] * p0);
+          if (c0 + u < s) out[lane == 0 ? c0 + u : s - 1 - c0 - u] = make_double2(p1, p2);
+          p0 = p1;
+          p1 = p2;
+        }
+        if (fabs(p0) < 0x1p-300 && fabs(p1) < 0x1p-300) {
           p0 *= 0x1p300;
           p1 *= 0x1p300;
         }
@@ -1050,32 +1162,38 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
         kmin = k;
       }
     }
+    // z = 1 at the twist, a running product away from it on either side (the
+    // factors on the other side are one)
+    double zl[2], zu[2];
 #pragma unroll
-    for (int c = 0; c < 2; ++c)
-      if (lane + 32 * c < s) Lp[lane + 32 * c] = make_double2(lo_r[c], up_r[c]);
-    __syncwarp();
-    if (lane < 2) {
-      double z = 1.0;
-      if (lane == 0) {
-        V[kmin * ld + q] = 1.0;
-#pragma unroll 4
-        for (int i = kmin - 1; i >= 0; --i) {
-          z *= Lp[i].x;
-          V[i * ld + q] = z;
-        }
-      } else {
-#pragma unroll 4
-        for (int i = kmin + 1; i < s; ++i) {
-          z *= Lp[i].y;
-          V[i * ld + q] = z;
-        }
+    for (int c = 0; c < 2; ++c) {
+      zl[c] = lane + 32 * c < kmin ? lo_r[c] : 1.0;
+      zu[c] = lane + 32 * c > kmin && lane + 32 * c < s ? up_r[c] : 1.0;
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (c == 1 && s <= 32) break;
+        const double dn = __shfl_down_sync(0xffffffffu, zl[c], o), up = __shfl_up_sync(0xffffffffu, zu[c], o);
+        if (lane + o < 32) zl[c] *= dn;
+        if (lane >= o) zu[c] *= up;
       }
     }
-    __syncwarp();
+    if (s > 32) {
+      zl[0] *= __shfl_sync(0xffffffffu, zl[1], 0);
+      zu[1] *= __shfl_sync(0xffffffffu, zu[0], 31);
+    }
     double n2 = 0.0;
-    for (int i = lane; i < s; i += 32) n2 = fma(V[i * ld + q], V[i * ld + q], n2);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      zl[c] *= zu[c];
+      if (lane + 32 * c < s) n2 = fma(zl[c], zl[c], n2);
+    }
     n2 = 1.0 / sqrt(warp_sum(n2));
-    for (int i = lane; i < s; i += 32) V[i * ld + q] *= n2;
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if (lane + 32 * c < s) V[(lane + 32 * c) * ld + q] = zl[c] * n2;
     if (lane == 0) th[q] = t;
   }
   __syncthreads();
@@ -1125,22 +1243,92 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
     if (!(fabs(r) <= 2e-13)) off = 1;
   }
   if (__syncthreads_or(off)) return false;
-  // ---- back-transformation, one warp a vector ----
-  for (int q = warp; q < nsel; q += nw) {
-    double z0 = lane < s ? V[lane * ld + q] : 0.0;
-    double z1 = lane + 32 < s ? V[(lane + 32) * ld + q] : 0.0;
+  // ---- back-transformation: eight lanes a vector, element i on lane i % 8 ----
+  for (int q0 = warp * 4; q0 < nsel; q0 += nw * 4) {
+    const int g = lane & 7, q = q0 + (lane >> 3);
+    const bool mine = q < nsel;
+    double z[kTriMax / 8];
+#pragma unroll
+    for (int c = 0; c < kTriMax / 8; ++c) z[c] = (mine && g + 8 * c < s) ? V[(g + 8 * c) * ld + q] : 0.0;
+#pragma unroll 1
     for (int j = s - 3; j >= 0; --j) {
-      const double v0 = (lane > j && lane < s) ? A[j * ld + lane] : 0.0;
-      const double v1 = (lane + 32 > j && lane + 32 < s) ? A[j * ld + lane + 32] : 0.0;
-      const double c = tau[j] * warp_sum(fma(v0, z0, v1 * z1));
-      z0 = fma(-c, v0, z0);
-      z1 = fma(-c, v1, z1);
+      double v[kTriMax / 8], t0 = 0.0, t1 = 0.0;
+#pragma unroll
+      for (int c = 0; c < kTriMax / 8; ++c) {
+        const int i = g + 8 * c;
+        v[c] = (i > j && i < s) ? A[j * ld + i] : 0.0;
+        if (c & 1) t1 = fma(v[c], z[c], t1);
+        else t0 = fma(v[c], z[c], t0);
+      }
+      t0 += t1;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+      t0 *= tau[j];
+#pragma unroll
+      for (int c = 0; c < kTriMax / 8; ++c) z[c] = fma(-t0, v[c], z[c]);
     }
-    if (lane < s) V[lane * ld + q] = z0;
-    if (lane + 32 < s) V[(lane + 32) * ld + q] = z1;
-    if (lane == 0) theta[q] = th[q] * sscale;
+#pragma unroll
+    for (int c = 0; c < kTriMax / 8; ++c)
+      if (mine && g + 8 * c < s) V[(g + 8 * c) * ld + q] = z[c];
+    if (mine && g == 0) theta[q] = th[q] * sscale;
   }
   __syncthreads();
+  return true;
+}
+
+// In-place elimination of [B | I] (B symmetric positive definite, ld) to
+// M = L^-1, B = L L^T: rows in registers (warp w holds rows w + q NW, lane l
+// columns l and, WIDE, l + 32; column c <= j of row i already holds L^-1 at
+// pivot j, the rest the trailing matrix), the pivot row published in shared
+// memory, one barrier a pivot.  False when a pivot is <= tol.
+template <int NW, int RW, bool WIDE>
+__device__ bool cta_inverse_cholesky(double* B, int s, int ld, double tol, double (*rowbuf)[kTriMax]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int l1 = lane + 32;
+  double a0[RW], a1[RW];
+#pragma unroll
+  for (int q = 0; q < RW; ++q) {
+    const int r = warp + q * NW;
+    a0[q] = (r < s && lane < s) ? B[r * ld + lane] : 0.0;
+    a1[q] = (WIDE && r < s && l1 < s) ? B[r * ld + l1] : 0.0;
+  }
+  if (warp == 0) {
+    rowbuf[0][lane] = a0[0];
+    if (WIDE && l1 < kTriMax) rowbuf[0][l1] = a1[0];
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int j = 0; j < s; ++j) {
+    const double* row = rowbuf[j & 1];
+    const double piv = row[j];
+    if (!(piv > tol)) return false;  // the same value in every thread
+    const double inv = 1.0 / piv;
+    const double r0 = row[lane], r1 = WIDE && l1 < kTriMax ? row[l1] : 0.0;
+#pragma unroll
+    for (int q = 0; q < RW; ++q) {
+      const int i = warp + q * NW;
+      const double f = __shfl_sync(0xffffffffu, !WIDE || j < 32 ? a0[q] : a1[q], j & 31) * inv;
+      if (i > j) {
+        a0[q] = lane == j ? -f : fma(-f, r0, a0[q]);
+        if (WIDE) a1[q] = l1 == j ? -f : fma(-f, r1, a1[q]);
+        if (i == j + 1) {
+          double* nr = rowbuf[(j + 1) & 1];
+          nr[lane] = a0[q];
+          if (WIDE && l1 < kTriMax) nr[l1] = a1[q];
+        }
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int q = 0; q < RW; ++q) {
+    const int i = warp + q * NW;
+    const double piv = __shfl_sync(0xffffffffu, !WIDE || i < 32 ? a0[q] : a1[q], i & 31);
+    if (i >= s) break;
+    const double f = 1.0 / sqrt(piv);
+    if (lane < s) B[i * ld + lane] = lane < i ? a0[q] * f : (lane == i ? f : 0.0);
+    if (WIDE && l1 < s) B[i * ld + l1] = l1 < i ? a1[q] * f : (l1 == i ? f : 0.0);
+  }
   return true;
 }
 
@@ -1154,7 +1342,7 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
 __device__ bool cta_rr_general_par(const double* gb, const double* ga, int P, const int* idx, int s, int nsel,
                                    int largest, double chol_tol, SmallSmem sm, double* dsc, double* theta_out,
                                    double* red, int* order, int* sflag) {
-  __shared__ double lsq[3 * MAXM];  // 1 / sqrt of the pivots
+  __shared__ double rowbuf[2][kTriMax];
   const int ld = sm.ld;
   const int nt = blockDim.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nt >> 5;
@@ -1176,28 +1364,11 @@ __device__ bool cta_rr_general_par(const double* gb, const double* ga, int P, co
     }
   }
   __syncthreads();
-  // ---- elimination of [B | I]: column c <= j of row i holds L^-1, the rest B ----
-  for (int j = 0; j < s; ++j) {
-    const double piv = sm.B[j * ld + j];
-    if (!(piv > chol_tol)) return false;  // the same value in every thread
-    const double inv = 1.0 / piv;
-    const double r0 = sm.B[j * ld + min(lane, s - 1)];
-    const double r1 = s > 32 ? sm.B[j * ld + min(lane + 32, s - 1)] : 0.0;
-    for (int i = j + 1 + warp; i < s; i += nw) {
-      double* row = sm.B + i * ld;
-      const double f = row[j] * inv;
-      __syncwarp();
-      if (lane < s) row[lane] = lane == j ? -f : fma(-f, r0, row[lane]);
-      if (lane + 32 < s) row[lane + 32] = lane + 32 == j ? -f : fma(-f, r1, row[lane + 32]);
-    }
-    __syncthreads();
-  }
-  for (int i = threadIdx.x; i < s; i += nt) lsq[i] = 1.0 / sqrt(sm.B[i * ld + i]);
-  __syncthreads();
-  for (int i = warp; i < s; i += nw) {  // M = diag(1 / l_ii) (unit lower inverse)
-    const double f = lsq[i];
-    for (int j = lane; j < s; j += 32) sm.B[i * ld + j] = j < i ? sm.B[i * ld + j] * f : (j == i ? f : 0.0);
-  }
+  // ---- M = L^-1 in place of B ----
+  const bool spd = nt == ST_WIDE ? cta_inverse_cholesky<ST_WIDE / 32, 3, true>(sm.B, s, ld, chol_tol, rowbuf)
+                   : s <= 12     ? cta_inverse_cholesky<ST / 32, 3, false>(sm.B, s, ld, chol_tol, rowbuf)
+                                 : cta_inverse_cholesky<ST / 32, 8, false>(sm.B, s, ld, chol_tol, rowbuf);
+  if (!spd) return false;
   __syncthreads();
   // ---- C = M A M^T: Y = M A, kept transposed in Z with row r rotated by r
   // (both the transposed store and the row reads are free of bank conflicts),
@@ -1205,43 +1376,65 @@ __device__ bool cta_rr_general_par(const double* gb, const double* ga, int P, co
   for (int i0 = warp; i0 < s; i0 += 3 * nw) {
     const int i1 = min(i0 + nw, s - 1), i2 = min(i0 + 2 * nw, s - 1);
     const double *m0 = sm.B + i0 * ld, *m1 = sm.B + i1 * ld, *m2 = sm.B + i2 * ld;
-    for (int c = lane; c < s; c += 32) {
-      double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-#pragma unroll 4
-      for (int k = 0; k <= i2; ++k) {
-        const double a = sm.A[k * ld + c];
-        v0 = fma(m0[k], a, v0);
-        v1 = fma(m1[k], a, v1);
-        v2 = fma(m2[k], a, v2);
+    double v0[2] = {0.0, 0.0}, v1[2] = {0.0, 0.0}, v2[2] = {0.0, 0.0};
+    const int c0 = min(lane, s - 1), c1 = min(lane + 32, s - 1);
+#pragma unroll 2
+    for (int k = 0; k <= i2; ++k) {
+      const double b0 = m0[k], b1 = m1[k], b2 = m2[k];
+      const double a = sm.A[k * ld + c0];
+      v0[0] = fma(b0, a, v0[0]);
+      v1[0] = fma(b1, a, v1[0]);
+      v2[0] = fma(b2, a, v2[0]);
+      if (s > 32) {
+        const double h = sm.A[k * ld + c1];
+        v0[1] = fma(b0, h, v0[1]);
+        v1[1] = fma(b1, h, v1[1]);
+        v2[1] = fma(b2, h, v2[1]);
       }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int c = lane + 32 * t;
+      if (c >= s) break;
       double* z = sm.Z + c * ld;
-      z[i0 + c < s ? i0 + c : i0 + c - s] = v0;
-      if (i0 + nw < s) z[i1 + c < s ? i1 + c : i1 + c - s] = v1;
-      if (i0 + 2 * nw < s) z[i2 + c < s ? i2 + c : i2 + c - s] = v2;
+      z[i0 + c < s ? i0 + c : i0 + c - s] = v0[t];
+      if (i0 + nw < s) z[i1 + c < s ? i1 + c : i1 + c - s] = v1[t];
+      if (i0 + 2 * nw < s) z[i2 + c < s ? i2 + c : i2 + c - s] = v2[t];
     }
   }
   __syncthreads();
   for (int i0 = warp; i0 < s; i0 += 3 * nw) {
     const int i1 = min(i0 + nw, s - 1), i2 = min(i0 + 2 * nw, s - 1);
     const double *m0 = sm.B + i0 * ld, *m1 = sm.B + i1 * ld, *m2 = sm.B + i2 * ld;
-    for (int c = lane; c < s; c += 32) {
-      double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-#pragma unroll 4
-      for (int k = 0; k <= i2; ++k) {
-        const double y = sm.Z[k * ld + (c + k < s ? c + k : c + k - s)];
-        v0 = fma(m0[k], y, v0);
-        v1 = fma(m1[k], y, v1);
-        v2 = fma(m2[k], y, v2);
+    double v0[2] = {0.0, 0.0}, v1[2] = {0.0, 0.0}, v2[2] = {0.0, 0.0};
+    const int c0 = min(lane, s - 1), c1 = min(lane + 32, s - 1);
+#pragma unroll 2
+    for (int k = 0; k <= i2; ++k) {
+      const double b0 = m0[k], b1 = m1[k], b2 = m2[k];
+      const double y = sm.Z[k * ld + (c0 + k < s ? c0 + k : c0 + k - s)];
+      v0[0] = fma(b0, y, v0[0]);
+      v1[0] = fma(b1, y, v1[0]);
+      v2[0] = fma(b2, y, v2[0]);
+      if (s > 32) {
+        const double h = sm.Z[k * ld + (c1 + k < s ? c1 + k : c1 + k - s)];
+        v0[1] = fma(b0, h, v0[1]);
+        v1[1] = fma(b1, h, v1[1]);
+        v2[1] = fma(b2, h, v2[1]);
       }
-      sm.A[i0 * ld + c] = v0;
-      sm.T[i0 * ld + c] = v0;
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int c = lane + 32 * t;
+      if (c >= s) break;
+      sm.A[i0 * ld + c] = v0[t];
+      sm.T[i0 * ld + c] = v0[t];
       if (i0 + nw < s) {
-        sm.A[i1 * ld + c] = v1;
-        sm.T[i1 * ld + c] = v1;
+        sm.A[i1 * ld + c] = v1[t];
+        sm.T[i1 * ld + c] = v1[t];
       }
       if (i0 + 2 * nw < s) {
-        sm.A[i2 * ld + c] = v2;
-        sm.T[i2 * ld + c] = v2;
+        sm.A[i2 * ld + c] = v2[t];
+        sm.T[i2 * ld + c] = v2[t];
       }
     }
   }
@@ -1250,7 +1443,7 @@ __device__ bool cta_rr_general_par(const double* gb, const double* ga, int P, co
   // on C where that route does not apply or its tests fail (pairs that agree
   // to rounding)
   bool direct = false;
-  if (s >= 3 && s * nsel <= 2 * nt) {
+  if (s >= 3 && s <= (nt == ST_WIDE ? kTriMax : 24) && s * nsel <= 2 * nt) {
     direct = cta_tri_select(sm.T, s, ld, nsel, largest, theta_out, sm.V, sm.W);
   }
   if (direct) {
@@ -1313,7 +1506,7 @@ __device__ bool rr_general(const double* gb, const double* ga, int P, const int*
       return warp_rr_general(gb, ga, P, idx, s, nsel, largest, chol_tol, sm.Z, sm.ld, sm.T, theta_out);
   }
   if constexpr (PAR) {
-    if (s <= 3 * MAXM)
+    if (s <= (NT == ST_WIDE ? 3 * MAXM : 32))
       return cta_rr_general_par(gb, ga, P, idx, s, nsel, largest, chol_tol, sm, dsc, theta_out, red, order, sflag);
   }
   return cta_rr_general(gb, ga, P, idx, s, nsel, largest, chol_tol, sm, dsc, theta_out, red, rc, rs, ra, rb, order,
