@@ -255,6 +255,42 @@ def test_dense_evd_tridiag_paths(gpu_ctx, monkeypatch, n, path):
         assert resid(p, vecs[:, j], vals[j]) < 1e-10
 
 
+@pytest.mark.parametrize("n", [3, 4, 16, 17, 33, 64, 65, 129, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 1537,
+                               2047, 2048])
+def test_dense_evd_direct_edges(gpu_ctx, n):
+    """Cluster and cooperative tridiagonalisation, direct tridiagonal pairs and
+    the blocked back-transformation at the edges of their ranges against
+    LAPACK: a connected weighted graph's Laplacian (distinct pairs), and the
+    same matrix twice on the diagonal (every eigenvalue double: the direct
+    route's test has to fail over to inverse iteration).  The bound is the
+    backward error n eps |A| (4.6e-13 at n = 2048) with room for a constant."""
+    import spectral_init_b200 as si
+    rng = np.random.default_rng(n)
+
+    def lap_of(m):
+        rows = np.r_[np.arange(m - 1), rng.integers(0, m, 3 * m)]
+        cols = np.r_[np.arange(1, m), rng.integers(0, m, 3 * m)]
+        a = sp.coo_matrix((rng.uniform(0.1, 1.0, rows.size), (rows, cols)), shape=(m, m)).tocsr()
+        a = (a + a.T).tolil()
+        a.setdiag(0.0)
+        a = a.tocsr()
+        a.eliminate_zeros()
+        dinv = 1.0 / np.sqrt(np.asarray(a.sum(axis=1)).ravel())
+        return sp.identity(m) - sp.diags(dinv) @ a @ sp.diags(dinv)
+
+    mats = [lap_of(n).tocsr()]
+    if n >= 16 and n % 2 == 0:
+        half = lap_of(n // 2)
+        mats.append(sp.block_diag([half, half]).tocsr())
+    k = min(5, n)
+    for lap in mats:
+        vals, vecs = si.dense_evd(lap, k, ctx=gpu_ctx)
+        want = np.linalg.eigvalsh(lap.toarray())[:k]
+        assert np.max(np.abs(vals - want)) < 1e-11
+        assert np.max(np.abs(vecs.T @ vecs - np.eye(k))) < 1e-11
+        assert np.max(np.abs(lap @ vecs - vecs * vals)) < 1e-11
+
+
 # ---- LOBPCG with 8- and 16-column blocks (register-tiled Gram, four-column update) -------------
 @pytest.mark.parametrize("nc,block", [(5, 0), (5, 7), (8, 0), (8, 10), (12, 0)])
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
