@@ -181,7 +181,7 @@ __global__ void k_tri_last(const double* A, int n, double* d, double* e, double*
 // c = tid + q * 256.  A step is one exchange between the CTAs:
 //   pass    every CTA applies the previous step's A -= v w^T + w v^T to its
 //           rows r > j and, in the same pass over shared memory, forms
-//           p_r = (A v_j)_r; it also picks up a_r = A(r, j + 1);
+//           p_r = (A v_j)_r; a_r = A(r, j + 1) is then up to step j - 1;
 //   gather  every CTA publishes (p_r, a_r) of its rows and reads everybody's;
 //   local   every CTA then knows p and column j + 1 and forms for itself
 //           K = tau^2 (p.v) / 2, w = tau p - K v, the updated column
@@ -257,18 +257,21 @@ __device__ __forceinline__ double warp_sum16(double (&a)[CT_CHUNK], int lane) {
 
 template <int CMAX, bool CLUSTER>
 __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
-  extern __shared__ __align__(16) double rows[];  // [R][n], then (cluster) [2][n] pairs
+  // [R][n + 1] (cluster: [R + 1], a spare row), then (cluster) [2][n] pairs
+  extern __shared__ __align__(16) double rows[];
   __shared__ double pr[CT_WARPS][CT_RMAX];        // row products, a partial per warp
-  __shared__ double vr[CT_RMAX], wr[CT_RMAX], ar[CT_RMAX];
+  __shared__ double vr[CT_RMAX + CT_CHUNK], wr[CT_RMAX + CT_CHUNK];
   __shared__ __align__(16) double red_s[CT_WARPS], red_d[CT_WARPS];
   __shared__ double s_alpha, s_p1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = p.n, G = p.G, R = p.R, b = blockIdx.x;
-  double2* pairs = reinterpret_cast<double2*>(rows + ((static_cast<size_t>(R) * n + 1) & ~size_t(1)));
-  for (int l = 0; l < R; ++l) {
+  const int ns = n + 1;
+  double2* pairs = reinterpret_cast<double2*>(rows + ((static_cast<size_t>(R + 1) * ns + 1) & ~size_t(1)));
+  for (int l = 0; l < (CLUSTER ? R + 1 : R); ++l) {
     const int r = l * G + b;
-    if (r >= n) break;
-    for (int c = tid; c < n; c += CT_THREADS) rows[l * n + c] = p.A[static_cast<int64_t>(r) * n + c];
+    const bool held = l < R && r < n;
+    for (int c = tid; c <= n; c += CT_THREADS)
+      rows[l * ns + c] = held && c < n ? p.A[static_cast<int64_t>(r) * n + c] : 0.0;
   }
   // x: column j from the diagonal down; v, w of the previous step; v of this one
   double x[CMAX], vp[CMAX], wp[CMAX], vc[CMAX];
@@ -279,7 +282,15 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
     vp[q] = 0.0;
     wp[q] = 0.0;
   }
-  if (tid < CT_RMAX) {
+  int slot[CMAX];  // where this CTA keeps row c, -1: it does not
+  int col[CMAX];
+#pragma unroll
+  for (int q = 0; q < CMAX; ++q) {
+    const int c = tid + q * CT_THREADS;
+    col[q] = min(c, n);
+    slot[q] = c < n && c % G == b ? c / G : -1;
+  }
+  if (tid < CT_RMAX + CT_CHUNK) {
     vr[tid] = 0.0;
     wr[tid] = 0.0;
   }
@@ -304,41 +315,69 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
       const double2 t = *reinterpret_cast<const double2*>(red_s + w);
       sigma += t.x + t.y;
     }
+    // H = I - tau v v^T, v = S (alpha - beta, x_{j+2}, ..) unnormalised: its
+    // division is not needed before w.  S, a power of two, keeps the products
+    // of a nearly zero column out of the underflow range.
+    const double S = sigma < 0x1p-700 ? 0x1p400 : 1.0;
     const double alpha = s_alpha;
-    double tau = 0.0, beta = alpha, scal = 0.0;
+    double beta = alpha, v1 = 0.0, tau_inv = 0.0;
     if (sigma > 0.0) {
       const double nrm = sqrt(fma(alpha, alpha, sigma));
       beta = alpha >= 0.0 ? -nrm : nrm;
-      tau = (beta - alpha) / beta;
-      scal = 1.0 / (alpha - beta);
+      v1 = (alpha - beta) * S;
+      tau_inv = -(beta * S) * v1;
     }
 #pragma unroll
     for (int q = 0; q < CMAX; ++q) {
       const int c = tid + q * CT_THREADS;
-      vc[q] = c == j + 1 ? 1.0 : (c > j + 1 ? x[q] * scal : 0.0);  // x is zero past the end
+      vc[q] = c == j + 1 ? v1 : (c > j + 1 ? x[q] * S : 0.0);  // x is zero past the end
     }
     // pass: slots below l0 hold finished rows (r <= j)
     const int l0 = j >= b ? (j - b) / G + 1 : 0;
     const int live = (n - b + G - 1) / G;  // slots that hold a row
-    for (int lb = l0; lb < live; lb += CT_CHUNK) {
+    bool on[CMAX], any = false;
+#pragma unroll
+    for (int q = 0; q < CMAX; ++q) {
+      const int c = warp * 32 + q * CT_THREADS;  // the group's first column
+      on[q] = c + 31 > j && c < n;
+      any = any || on[q];
+    }
+    if (!any && lane < CT_RMAX) pr[warp][lane] = 0.0;
+    for (int lb = any ? l0 : live; lb < live; lb += CT_CHUNK) {
       double acc[CT_CHUNK];
+      // Finished columns need no guard (v and w are zero there); a warp skips
+      // a column group that is finished as a whole, and columns past the end
+      // go to a pad column.  GR rows are loaded together: the stores of one
+      // row could alias the loads of the next as far as the compiler knows;
+      // with two columns a thread, rows past the end go to a spare row.
+      constexpr int GR = CMAX == 2 ? 4 : 1;
 #pragma unroll
-      for (int i = 0; i < CT_CHUNK; ++i) acc[i] = 0.0;
+      for (int g = 0; g < CT_CHUNK; g += GR) {
 #pragma unroll
-      for (int q = 0; q < CMAX; ++q) {
-        const int c = tid + q * CT_THREADS;
-        if (c > j && c < n) {
-          double* col = rows + lb * n + c;
+        for (int i = 0; i < GR; ++i) acc[g + i] = 0.0;
+        if (lb + g >= live) continue;
+        double a[GR][CMAX];
+        double* row[GR];
 #pragma unroll
-          for (int i = 0; i < CT_CHUNK; ++i) {
-            if (lb + i < live) {
-              const double a = fma(-vr[lb + i], wp[q], fma(-wr[lb + i], vp[q], col[i * n]));
-              col[i * n] = a;
-              acc[i] = fma(a, vc[q], acc[i]);
-              if (c == j + 1) ar[lb + i] = a;
-            }
+        for (int i = 0; i < GR; ++i) {
+          row[i] = rows + min(lb + g + i, GR > 1 ? live : R - 1) * ns;
+#pragma unroll
+          for (int q = 0; q < CMAX; ++q) a[i][q] = on[q] ? row[i][col[q]] : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < GR; ++i) {
+          const double nv = -vr[lb + g + i], nw = -wr[lb + g + i];
+#pragma unroll
+          for (int q = 0; q < CMAX; ++q) {
+            a[i][q] = fma(nv, wp[q], fma(nw, vp[q], a[i][q]));
+            acc[g + i] = fma(a[i][q], vc[q], acc[g + i]);
           }
         }
+#pragma unroll
+        for (int i = 0; i < GR; ++i)
+#pragma unroll
+          for (int q = 0; q < CMAX; ++q)
+            if (on[q]) row[i][col[q]] = a[i][q];
       }
       const double sum = warp_sum16(acc, lane);
       if ((lane & 1) == 0 && lb + (lane >> 1) < live) pr[warp][lb + (lane >> 1)] = sum;
@@ -346,20 +385,26 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
     __syncthreads();
     // publish own rows
     const uint64_t step = static_cast<uint64_t>(j) + 1;
-    if (l0 + tid < live) {
-      const int l = l0 + tid, r = l * G + b;
+    const int nl = live - l0;
+    if constexpr (CLUSTER) {
+      // a thread a (row, peer) pair
+      for (int t = tid; t < CT_RMAX * G; t += CT_THREADS) {
+        const int peer = t / CT_RMAX, l = l0 + (t & (CT_RMAX - 1));
+        if (l >= live) continue;
+        double sum = 0.0;
+#pragma unroll
+        for (int w = 0; w < CT_WARPS; ++w) sum += pr[w][l];
+        *cooperative_groups::this_cluster().map_shared_rank(pairs + (j & 1) * n + l * G + b, peer) =
+            make_double2(sum, rows[l * ns + j + 1]);
+      }
+    } else if (tid < nl) {
+      const int l = l0 + tid;
       double sum = 0.0;
 #pragma unroll
       for (int w = 0; w < CT_WARPS; ++w) sum += pr[w][l];
-      if constexpr (CLUSTER) {
-        double2* mine = pairs + (j & 1) * n + r;
-        for (int t = 0; t < G; ++t)
-          *cooperative_groups::this_cluster().map_shared_rank(mine, t) = make_double2(sum, ar[l]);
-      } else {
-        ulonglong2* out = p.words + (static_cast<size_t>(j & 1) * n + r) * 2;
-        st_word(out, sum, step);
-        st_word(out + 1, ar[l], step);
-      }
+      ulonglong2* out = p.words + (static_cast<size_t>(j & 1) * n + l * G + b) * 2;
+      st_word(out, sum, step);
+      st_word(out + 1, rows[l * ns + j + 1], step);
     }
     // gather
     double pc[CMAX], ac[CMAX];
@@ -383,28 +428,38 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
         ac[q] = 0.0;
         if (c > j && c < n) missing |= 1u << q;
       }
+      // Above 1024 columns a thread polls for its first column alone until that
+      // one is there: n 32-byte words a CTA and round, read while nothing has
+      // arrived, hold up the words being published (8.1 against 6.6 us a column
+      // at n = 1873; below, all columns from the start are faster, 4.1 against
+      // 5.2 us at n = 1000).
       uint64_t t0 = 0;
-      for (int tries = 0; missing != 0; ++tries) {
+      bool one = CMAX > 4;
+      while (missing != 0) {
+        const unsigned ask = one ? missing & (0u - missing) : missing;
         ulonglong2 wa[CMAX], wb[CMAX];
 #pragma unroll
         for (int q = 0; q < CMAX; ++q) {
-          if (missing >> q & 1u) {
+          if (ask >> q & 1u) {
             const ulonglong2* at = in + static_cast<size_t>(tid + q * CT_THREADS) * 2;
             wa[q] = ld_word(at);
             wb[q] = ld_word(at + 1);
           }
         }
+        unsigned got = 0;
 #pragma unroll
         for (int q = 0; q < CMAX; ++q) {
-          if ((missing >> q & 1u) && wa[q].y == step && wb[q].y == step) {
+          if ((ask >> q & 1u) && wa[q].y == step && wb[q].y == step) {
             pc[q] = __longlong_as_double(static_cast<long long>(wa[q].x));
             ac[q] = __longlong_as_double(static_cast<long long>(wb[q].x));
-            missing &= ~(1u << q);
+            got |= 1u << q;
           }
         }
-        if (missing != 0 && (tries & 15) == 0) {
+        missing &= ~got;
+        if (got != 0) one = false;
+        if (got == 0) {
           const uint64_t now = coop_ns();
-          if (tries == 0) t0 = now;
+          if (t0 == 0) t0 = now;
           if (now - t0 >= p.wait_ns || *reinterpret_cast<volatile int*>(p.err) != 0) {
             if (now - t0 >= p.wait_ns) atomicExch(p.err, 1);
             fail = 1;
@@ -414,15 +469,17 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
       }
     }
     // row j of A now belongs to the reflector (every CTA has long read its input)
-    if (owner) {
+    const double tau = tau_inv != 0.0 ? 1.0 / tau_inv : 0.0;
+    if (owner) {  // normalised to a first element of one, as the back-transformation reads it
+      const double inv = v1 != 0.0 ? 1.0 / v1 : 0.0;
 #pragma unroll
       for (int q = 0; q < CMAX; ++q) {
         const int c = tid + q * CT_THREADS;
-        if (c > j + 1 && c < n) p.A[static_cast<int64_t>(j) * n + c] = vc[q];
+        if (c > j + 1 && c < n) p.A[static_cast<int64_t>(j) * n + c] = vc[q] * inv;
       }
       if (tid == 0) {
         p.e[j] = beta;
-        p.tau[j] = tau;
+        p.tau[j] = tau * v1 * v1;
       }
     }
     // w and column j + 1
@@ -446,16 +503,15 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
       pv += t.x + t.y;
     }
     const double K = 0.5 * tau * tau * pv;
-    const double w1 = fma(tau, s_p1, -K);  // w_{j+1}; v_{j+1} = 1
+    const double w1 = fma(tau, s_p1, -K * v1);  // w_{j+1}
 #pragma unroll
     for (int q = 0; q < CMAX; ++q) {
-      const int c = tid + q * CT_THREADS;
       vp[q] = tau != 0.0 ? vc[q] : 0.0;
       wp[q] = tau != 0.0 ? fma(tau, pc[q], -K * vc[q]) : 0.0;
-      x[q] = tau != 0.0 ? ac[q] - fma(vp[q], w1, wp[q]) : ac[q];
-      if (c > j && c < n && c % G == b) {
-        vr[c / G] = vp[q];
-        wr[c / G] = wp[q];
+      x[q] = tau != 0.0 ? ac[q] - fma(vp[q], w1, wp[q] * v1) : ac[q];
+      if (slot[q] >= l0) {
+        vr[slot[q]] = vp[q];
+        wr[slot[q]] = wp[q];
       }
     }
   }
@@ -470,7 +526,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
       }
       if (c == n - 1) p.e[n - 2] = x[q];
     }
-    if ((n - 1) % G == b && c == n - 1) p.d[c] = fma(-2.0 * vp[q], wp[q], rows[(c / G) * n + c]);
+    if ((n - 1) % G == b && c == n - 1) p.d[c] = fma(-2.0 * vp[q], wp[q], rows[(c / G) * ns + c]);
   }
   if constexpr (CLUSTER) cooperative_groups::this_cluster().sync();  // no peer stores into a CTA that has left
 }
@@ -1391,7 +1447,8 @@ bool tridiag_cluster(const Exec& ex, const CoopTri& base) {
   p.G = 1;
   while (p.G < 16 && p.G * CT_CHUNK < n) p.G *= 2;
   p.R = ceil_div(n, p.G);
-  const size_t smem = sizeof(double) * ((static_cast<size_t>(p.R) * n + 1) & ~size_t(1)) + sizeof(double2) * 2 * n;
+  const size_t smem =
+      sizeof(double) * ((static_cast<size_t>(p.R + 1) * (n + 1) + 1) & ~size_t(1)) + sizeof(double2) * 2 * n;
   auto* kernel = k_tridiag_coop<2, true>;
   if (p.R > CT_RMAX || smem > static_cast<size_t>(smem_limit(ex.device, kernel))) return false;
   cudaLaunchConfig_t cfg{};
@@ -1436,7 +1493,7 @@ bool tridiag_single(const Exec& ex, double* A, int n, double* d, double* e, doub
   G = std::min({G, n, ex.sms});
   const int R = ceil_div(n, G);
   G = ceil_div(n, R);
-  const size_t smem = sizeof(double) * static_cast<size_t>(R) * n;
+  const size_t smem = sizeof(double) * static_cast<size_t>(R) * (n + 1);
   auto* kernel = n <= 4 * CT_THREADS ? k_tridiag_coop<4, false> : k_tridiag_coop<CT_CMAX, false>;
   if (R > CT_RMAX || smem > static_cast<size_t>(smem_limit(ex.device, kernel))) return false;
   int occ = 0;

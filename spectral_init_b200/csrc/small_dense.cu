@@ -813,7 +813,7 @@ struct Reflector {
 };
 __device__ __forceinline__ Reflector make_reflector(double alpha, double sigma) {
   Reflector r{alpha, 0.0, 0.0};
-  if (sigma > 0.0) {
+  if (sigma > 0x1p-930) {  // below, tau_inv would underflow: entries of 1e-140 are zeros here
     const double nrm = sqrt(fma(alpha, alpha, sigma));
     r.beta = alpha >= 0.0 ? -nrm : nrm;
     r.v1 = alpha - r.beta;
