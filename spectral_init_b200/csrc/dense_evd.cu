@@ -189,8 +189,8 @@ __global__ void k_tri_last(const double* A, int n, double* d, double* e, double*
 // The exchange is what bounds a step (the pass reads and writes at most
 // 200 KB of shared memory a CTA, on average a third of that), and one is what
 // it takes: publishing the reflector and w each with a grid-wide wait of its
-// own measured 11 us a column at n = 1873, this TRICOOP us; one CTA alone
-// took 6.6 us a column at n = 150, a cluster here TRICLUS us.
+// own measured 11 us a column at n = 1873, this 6.1 us; one CTA alone
+// took 6.6 us a column at n = 150, a cluster here 2.1 us.
 //   CLUSTER (n <= kTriClusterMax): up to 16 CTAs of one thread-block cluster;
 //   a CTA stores its pairs into every peer's shared memory, the exchange is
 //   one cluster barrier.  Small solves leave the other SMs to concurrent ones.
@@ -406,6 +406,24 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
       st_word(out, sum, step);
       st_word(out + 1, rows[l * ns + j + 1], step);
     }
+    const double tau = tau_inv != 0.0 ? 1.0 / tau_inv : 0.0;
+    // Row j of A takes the reflector, normalised to a first element of one as
+    // the back-transformation reads it, while the other CTAs' words are on
+    // their way (row 0, which every CTA read at the start, after they came).
+    auto keep_reflector = [&] {
+      if (!owner) return;
+      const double inv = v1 != 0.0 ? 1.0 / v1 : 0.0;
+#pragma unroll
+      for (int q = 0; q < CMAX; ++q) {
+        const int c = tid + q * CT_THREADS;
+        if (c > j + 1 && c < n) p.A[static_cast<int64_t>(j) * n + c] = vc[q] * inv;
+      }
+      if (tid == 0) {
+        p.e[j] = beta;
+        p.tau[j] = tau * v1 * v1;
+      }
+    };
+    if (j > 0) keep_reflector();
     // gather
     double pc[CMAX], ac[CMAX];
     int fail = 0;
@@ -428,36 +446,28 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
         ac[q] = 0.0;
         if (c > j && c < n) missing |= 1u << q;
       }
-      // Above 1024 columns a thread polls for its first column alone until that
-      // one is there: n 32-byte words a CTA and round, read while nothing has
-      // arrived, hold up the words being published (8.1 against 6.6 us a column
-      // at n = 1873; below, all columns from the start are faster, 4.1 against
-      // 5.2 us at n = 1000).
       uint64_t t0 = 0;
-      bool one = CMAX > 4;
+      unsigned fails = 0;
       while (missing != 0) {
-        const unsigned ask = one ? missing & (0u - missing) : missing;
         ulonglong2 wa[CMAX], wb[CMAX];
 #pragma unroll
         for (int q = 0; q < CMAX; ++q) {
-          if (ask >> q & 1u) {
+          if (missing >> q & 1u) {
             const ulonglong2* at = in + static_cast<size_t>(tid + q * CT_THREADS) * 2;
             wa[q] = ld_word(at);
             wb[q] = ld_word(at + 1);
           }
         }
-        unsigned got = 0;
 #pragma unroll
         for (int q = 0; q < CMAX; ++q) {
-          if ((ask >> q & 1u) && wa[q].y == step && wb[q].y == step) {
+          if ((missing >> q & 1u) && wa[q].y == step && wb[q].y == step) {
             pc[q] = __longlong_as_double(static_cast<long long>(wa[q].x));
             ac[q] = __longlong_as_double(static_cast<long long>(wb[q].x));
-            got |= 1u << q;
+            missing &= ~(1u << q);
           }
         }
-        missing &= ~got;
-        if (got != 0) one = false;
-        if (got == 0) {
+        // the clock and the error word cost as much as a poll: every 64 rounds
+        if (missing != 0 && ((++fails & 63u) == 0 || p.wait_ns == 0)) {
           const uint64_t now = coop_ns();
           if (t0 == 0) t0 = now;
           if (now - t0 >= p.wait_ns || *reinterpret_cast<volatile int*>(p.err) != 0) {
@@ -468,20 +478,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
         }
       }
     }
-    // row j of A now belongs to the reflector (every CTA has long read its input)
-    const double tau = tau_inv != 0.0 ? 1.0 / tau_inv : 0.0;
-    if (owner) {  // normalised to a first element of one, as the back-transformation reads it
-      const double inv = v1 != 0.0 ? 1.0 / v1 : 0.0;
-#pragma unroll
-      for (int q = 0; q < CMAX; ++q) {
-        const int c = tid + q * CT_THREADS;
-        if (c > j + 1 && c < n) p.A[static_cast<int64_t>(j) * n + c] = vc[q] * inv;
-      }
-      if (tid == 0) {
-        p.e[j] = beta;
-        p.tau[j] = tau * v1 * v1;
-      }
-    }
+    if (j == 0) keep_reflector();
     // w and column j + 1
     double dot = 0.0;
 #pragma unroll
@@ -543,7 +540,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
 // k_tri_polish then orthonormalises the k vectors and tests them; where two
 // wanted eigenvalues agree to rounding (a matrix that splits, multiplicities)
 // the test fails and k_tri_eig, whose inverse iteration handles those, runs
-// instead.  Measured at n = 1873, k = 4: TRIDIRECT us against 4.6 ms for
+// instead.  Measured at n = 1873, k = 4: 0.51 ms against 4.6 ms for
 // k_tri_eig alone.
 constexpr int kTdThreads = 128;
 constexpr int64_t kTriDirectMax = 2048;
@@ -1224,7 +1221,7 @@ __global__ void __launch_bounds__(BW_THREADS) k_backtransform_wy(const double* _
 // thread owns rows tid + q * 512) and the next block's rows already in flight,
 // so the reflectors are read once a vector and a block costs two barriers.
 // Forming T on the way, by one thread, took most of k_backtransform_wy's 26 us
-// a block at n = 1873; this takes BCOLS us.
+// a block at n = 1873; this takes 2.2 us.
 constexpr int BC_THREADS = 512;
 constexpr int BC_RPT = 4;
 constexpr int kBcMax = BC_THREADS * BC_RPT;
