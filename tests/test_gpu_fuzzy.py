@@ -55,3 +55,38 @@ def test_fuzzy_graph_matches_oracle_on_a_larger_cloud(gpu_ctx):
     assert np.array_equal(g.indptr, ref.indptr) and np.array_equal(g.indices, ref.indices)
     assert np.allclose(g.data, ref.data, rtol=2e-6, atol=1e-7)
     assert (g != g.T).nnz == 0
+
+
+@pytest.mark.parametrize("n,d,k", [(2, 1, 1), (17, 3, 16), (64, 16, 5), (65, 17, 17), (129, 1, 32), (700, 50, 15),
+                                   (4097, 33, 16)])
+def test_knn_tile_edges_and_ties(gpu_ctx, n, d, k):
+    """Exact neighbours at the edges of query, candidate and feature tiles.
+    Integer coordinates: squared distances are exact and full of ties, which
+    go to the smaller index."""
+    import spectral_init_b200 as si
+    rng = np.random.default_rng(n + d)
+    x = rng.integers(0, 4, (n, d)).astype(np.float64)
+    _, (idx, dist, _, _) = si.fuzzy_graph(x, k, ctx=gpu_ctx, return_stages=True)
+    sq = (x * x).sum(1)
+    for s in range(0, n, 512):
+        d2 = sq[s:s + 512, None] + sq[None, :] - 2.0 * (x[s:s + 512] @ x.T)  # exact in f64
+        d2[np.arange(d2.shape[0]), np.arange(s, s + d2.shape[0])] = np.inf
+        want = np.argsort(d2, axis=1, kind="stable")[:, :k]
+        assert np.array_equal(idx[s:s + 512], want)
+        assert np.array_equal(dist[s:s + 512], np.sqrt(np.take_along_axis(d2, want, 1)).astype(np.float32))
+
+
+def test_fuzzy_graph_with_a_hub(gpu_ctx):
+    """Points in random directions around one centre, which is everybody's
+    nearest neighbour: its row is far longer than a warp sorts."""
+    import spectral_init_b200 as si
+    rng = np.random.default_rng(11)
+    v = rng.normal(size=(1500, 40))
+    x = np.concatenate([np.zeros((1, 40)), v / np.linalg.norm(v, axis=1, keepdims=True)
+                        * rng.uniform(1.0, 1.2, (1500, 1))])
+    g = si.fuzzy_graph(x, 5, ctx=gpu_ctx)
+    ref = F.fuzzy_graph(x, 5)
+    ref.sort_indices()
+    assert np.max(np.diff(g.indptr)) > 1000
+    assert np.array_equal(g.indptr, ref.indptr) and np.array_equal(g.indices, ref.indices)
+    assert np.allclose(g.data, ref.data, rtol=2e-6, atol=1e-7)
