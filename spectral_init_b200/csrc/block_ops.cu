@@ -246,151 +246,101 @@ __global__ void __launch_bounds__(G4_THREADS) k_gram4(const XT* __restrict__ X, 
   }
 }
 
-// Task-split Gram of a 4-column LOBPCG iteration.  Only the upper triangles
-// of S^T S and S^T AS are needed (156 of the 288 products a row of [S AS]
-// offers), so each of the CTA's four warps owns one share and computes it for
-// every row, one row per lane:
-//   warp 0: X^T [X R P]      (i in X, j >= i)    42 products from 12 values
-//   warp 1: [R P]^T [R P]    (i in R P, j >= i)  36 products from  8 values
-//   warp 2: X^T [AX AR AP]   (i in X, j >= i)    42 products from 16 values
-//   warp 3: [R P]^T [AR AP]  (i in R P, j >= i)  36 products from 16 values
-// A tile of 128 rows of the six blocks is loaded with coalesced 16-byte loads
-// (one warp reads 32 consecutive rows of one block), converted to f64 once
-// and stored with a row stride of 25 doubles, so a warp's 32 rows of one
-// column fall in distinct banks.  Accumulators stay in registers across all
-// tiles of the CTA; at the end each warp sums its lanes and the CTA writes
-// one 288-entry partial (the k_gram4 layout, unused entries zero) that
-// k_gram4_reduce adds in CTA order.
-constexpr int GT_TR = 128;
-constexpr int GT_STRIDE = 25;
-constexpr int GT_THREADS = 128;
+// Gram of a 4-column LOBPCG iteration on the FP64 matrix instruction
+// (mma.m8n8k4: A 8 x 4, B 4 x 8, accumulators 8 x 8).  With four rows of S as
+// the k dimension a lane's element of S^T (column lane / 4, row lane % 4) is
+// also its element of S, so one 8-byte load per lane is an operand on both
+// sides, straight from global memory: no shared memory, no conversion pass.
+// The six blocks as three column octets f0 = [X R], f1 = [P AP], f2 = [AX AR]
+// give every product of the two upper triangles in four instructions:
+//   f0 f0: XX XR RR;  f0 f1: XP RP X.AP R.AP;  f0 f2: X.AX X.AR R.AR;
+//   f1 f1: PP P.AP.
+// HBM is the bound (6 n ld s bytes).  The products used to be scalar, four
+// warps re-reading a 128-row tile from shared memory (60 reads a row): 48 us
+// f64 and 37 us f32 at n = 1M, 13.5 / 7.2 at n = 200k / 60k, against 27 and 39,
+// 6.3 / 3.9 here (floor 30 and 15 us at n = 1M; f32 is held by the instruction's
+// rate and the conversions, one unit for both).
+constexpr int GM_THREADS = 256;
+constexpr int GM_UNROLL = 4;  // groups of four rows in flight per warp
 
-template <int TASK>
-struct GramTask;
-template <>
-struct GramTask<0> { static constexpr int I0 = 0, I1 = 4, TOFF = 0, N = 42; };
-template <>
-struct GramTask<1> { static constexpr int I0 = 4, I1 = 12, TOFF = 0, N = 36; };
-template <>
-struct GramTask<2> { static constexpr int I0 = 0, I1 = 4, TOFF = 12, N = 42; };
-template <>
-struct GramTask<3> { static constexpr int I0 = 4, I1 = 12, TOFF = 12, N = 36; };
-
-template <int TASK>
-__device__ __forceinline__ void gram_task_row(const double* __restrict__ row, double (&acc)[42]) {
-  using T = GramTask<TASK>;
-  double s[12], t[12];
-#pragma unroll
-  for (int i = T::I0; i < 12; ++i) s[i] = row[i];
-  if constexpr (T::TOFF != 0) {
-#pragma unroll
-    for (int j = T::I0; j < 12; ++j) t[j] = row[T::TOFF + j];
-  }
-  int e = 0;
-#pragma unroll
-  for (int i = T::I0; i < T::I1; ++i) {
-#pragma unroll
-    for (int j = i; j < 12; ++j) {
-      const double tj = (T::TOFF != 0) ? t[j] : s[j];
-      acc[e] = fma(s[i], tj, acc[e]);
-      ++e;
-    }
-  }
-}
-
-template <int TASK>
-__device__ __forceinline__ void gram_task_store(const double (&acc)[42], double* red) {
-  using T = GramTask<TASK>;
-  int e = 0;
-#pragma unroll
-  for (int i = T::I0; i < T::I1; ++i) {
-#pragma unroll
-    for (int j = i; j < 12; ++j) {
-      red[i * 24 + T::TOFF + j] = acc[e];
-      ++e;
-    }
-  }
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
 }
 
 template <class XT>
-__global__ void __launch_bounds__(GT_THREADS) k_gram4t(const XT* __restrict__ X, const XT* __restrict__ R,
-                                                        const XT* __restrict__ P, const XT* __restrict__ AX,
-                                                        const XT* __restrict__ AR, const XT* __restrict__ AP,
-                                                        int64_t n, double* __restrict__ partial,
-                                                        const int* __restrict__ stop) {
+__global__ void __launch_bounds__(GM_THREADS) k_gram4m(const XT* __restrict__ X, const XT* __restrict__ R,
+                                                       const XT* __restrict__ P, const XT* __restrict__ AX,
+                                                       const XT* __restrict__ AR, const XT* __restrict__ AP,
+                                                       int64_t n, double* __restrict__ partial,
+                                                       const int* __restrict__ stop) {
   if (stop != nullptr && *stop != 0) return;
-  __shared__ double tile[GT_TR * GT_STRIDE];
-  __shared__ double red[288];
+  constexpr int NW = GM_THREADS / 32;
+  __shared__ double red[NW][4][64];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const XT* src[6] = {X, R, P, AX, AR, AP};
-  double acc[42];
+  const int col = lane >> 2, k = lane & 3;
+  const int64_t at = static_cast<int64_t>(k) * 4 + (col & 3);  // within four rows of a block
+  const XT* const p0 = (col < 4 ? X : R) + at;
+  const XT* const p1 = (col < 4 ? P : AP) + at;
+  const XT* const p2 = (col < 4 ? AX : AR) + at;
+  double c00[2] = {0.0, 0.0}, c01[2] = {0.0, 0.0}, c02[2] = {0.0, 0.0}, c11[2] = {0.0, 0.0};
+  const int64_t groups = (n + 3) / 4;
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * NW;
+  for (int64_t g0 = (static_cast<int64_t>(blockIdx.x) * NW + warp) * GM_UNROLL; g0 < groups;
+       g0 += warps * GM_UNROLL) {
+    XT f0[GM_UNROLL], f1[GM_UNROLL], f2[GM_UNROLL];
 #pragma unroll
-  for (int e = 0; e < 42; ++e) acc[e] = 0.0;
-  for (int e = tid; e < 288; e += GT_THREADS) red[e] = 0.0;
-  constexpr int EPC = 16 / sizeof(XT);  // elements per 16-byte load
-  constexpr int CPR = 4 / EPC;          // loads per (row, block)
-  const int64_t ntiles = (n + GT_TR - 1) / GT_TR;
-  for (int64_t tl = blockIdx.x; tl < ntiles; tl += gridDim.x) {
-    const int64_t row0 = tl * GT_TR;
-    // load: chunk c = (block b, half h, row r), rows fastest so a warp reads
-    // 32 consecutive rows of one block
-#pragma unroll 4
-    for (int c = tid; c < 6 * CPR * GT_TR; c += GT_THREADS) {
-      const int r = c % GT_TR;
-      const int bh = c / GT_TR;
-      const int b = bh / CPR, h = bh % CPR;
-      const int64_t row = row0 + r;
-      double v[EPC];
-      if (row < n) {
-        if constexpr (sizeof(XT) == 4) {
-          const float4 q = __ldcs(reinterpret_cast<const float4*>(src[b] + row * 4));
-          v[0] = q.x;
-          v[1] = q.y;
-          v[2] = q.z;
-          v[3] = q.w;
-        } else {
-          const double2 q = __ldcs(reinterpret_cast<const double2*>(src[b] + row * 4 + h * 2));
-          v[0] = q.x;
-          v[1] = q.y;
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < EPC; ++u) v[u] = 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < EPC; ++u) tile[r * GT_STRIDE + b * 4 + h * EPC + u] = v[u];
+    for (int u = 0; u < GM_UNROLL; ++u) {
+      const int64_t g = g0 + u;
+      const bool ok = g * 4 + k < n;
+      f0[u] = ok ? __ldcs(p0 + g * 16) : XT(0);
+      f1[u] = ok ? __ldcs(p1 + g * 16) : XT(0);
+      f2[u] = ok ? __ldcs(p2 + g * 16) : XT(0);
     }
-    __syncthreads();
-#pragma unroll 1
-    for (int r = lane; r < GT_TR; r += 32) {
-      const double* row = tile + r * GT_STRIDE;
-      switch (warp) {
-        case 0: gram_task_row<0>(row, acc); break;
-        case 1: gram_task_row<1>(row, acc); break;
-        case 2: gram_task_row<2>(row, acc); break;
-        default: gram_task_row<3>(row, acc); break;
-      }
+#pragma unroll
+    for (int u = 0; u < GM_UNROLL; ++u) {
+      const double a0 = static_cast<double>(f0[u]), a1 = static_cast<double>(f1[u]), a2 = static_cast<double>(f2[u]);
+      dmma(c00, a0, a0);
+      dmma(c01, a0, a1);
+      dmma(c02, a0, a2);
+      dmma(c11, a1, a1);
     }
-    __syncthreads();
   }
-  // sum each accumulator over the warp's lanes (fixed butterfly order)
+  // accumulator element t of a lane: row lane / 4, column 2 (lane % 4) + t
+  const int e = col * 8 + 2 * k;
 #pragma unroll
-  for (int e = 0; e < 42; ++e) {
-    double v = acc[e];
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    acc[e] = v;
-  }
-  if (lane == 0) {
-    switch (warp) {
-      case 0: gram_task_store<0>(acc, red); break;
-      case 1: gram_task_store<1>(acc, red); break;
-      case 2: gram_task_store<2>(acc, red); break;
-      default: gram_task_store<3>(acc, red); break;
-    }
+  for (int t = 0; t < 2; ++t) {
+    red[warp][0][e + t] = c00[t];
+    red[warp][1][e + t] = c01[t];
+    red[warp][2][e + t] = c02[t];
+    red[warp][3][e + t] = c11[t];
   }
   __syncthreads();
-  for (int e = tid; e < 288; e += GT_THREADS) partial[static_cast<int64_t>(blockIdx.x) * 288 + e] = red[e];
+  // one 288-entry partial per CTA, in the layout that k_gram4_reduce adds:
+  // entry i * 24 + j, i a column of S = [X R P], j of [S AS]
+  for (int o = tid; o < 288; o += GM_THREADS) {
+    const int i = o / 24, j = o - (o / 24) * 24;
+    const int bi = i >> 2, bj = j >> 2;  // blocks: X R P | X R P AX AR AP
+    int m = -1, r = 0, c = 0;
+    if (bi < 2) {  // X, R rows: octet 0
+      r = (bi & 1) * 4 + (i & 3);
+      if (bj < 2) { m = 0; c = (bj & 1) * 4 + (j & 3); }
+      else if (bj == 2) { m = 1; c = j & 3; }
+      else if (bj == 5) { m = 1; c = 4 + (j & 3); }
+      else { m = 2; c = (bj - 3) * 4 + (j & 3); }
+    } else if (bj == 2 || bj == 5) {  // P rows: octet 1
+      r = i & 3;
+      m = 3;
+      c = (bj == 2 ? 0 : 4) + (j & 3);
+    }
+    double sum = 0.0;
+    if (m >= 0) {
+#pragma unroll
+      for (int w = 0; w < NW; ++w) sum += red[w][m][r * 8 + c];
+    }
+    partial[static_cast<int64_t>(blockIdx.x) * 288 + o] = sum;
+  }
 }
 
 bool gram4_old_forced() {
@@ -683,6 +633,79 @@ __global__ void __launch_bounds__(256) k_lobpcg_update4(LobpcgBlocks<XT> b, cons
       b.P[o + j] = static_cast<XT>(active ? pn : 0.0);
       b.AP[o + j] = static_cast<XT>(active ? apn : 0.0);
     }
+  }
+}
+
+// The same update for f32 blocks: a thread takes a whole row, so an element is
+// converted to f64 once (four threads a row each convert the row: 116
+// conversions a row, and the unit does 16 a clock and SM, against 52 here).
+// n = 1M: 54 -> 36 us, floor 27 us (11 n ld s bytes).
+__global__ void __launch_bounds__(256, 2) k_lobpcg_update4_f32(LobpcgBlocks<float> b, const LobpcgCtrl* __restrict__ ctrl,
+                                                            int64_t n, int init_mode) {
+  __shared__ __align__(16) double sC[3][4][4];  // [block][input column][output column]
+  __shared__ double sLam[4];
+  __shared__ int sF[4];
+  if (threadIdx.x == 0) {
+    sF[0] = ctrl->done;
+    sF[1] = ctrl->copy_best;
+    sF[2] = ctrl->has_p;
+    sF[3] = ctrl->m;
+  }
+  if (threadIdx.x < 48) {
+    const int w = threadIdx.x / 16, r = (threadIdx.x / 4) % 4, c = threadIdx.x % 4;
+    const double* src = w == 0 ? ctrl->Cx : (w == 1 ? ctrl->Cr : ctrl->Cp);
+    sC[w][r][c] = src[r * MAXM + c];
+  }
+  if (threadIdx.x < 4) sLam[threadIdx.x] = ctrl->lam[threadIdx.x];
+  __syncthreads();
+  const int done = sF[0], copy_best = sF[1], use_p = sF[2], m = sF[3];
+  if (done && !copy_best) return;
+  auto rows = [](float* p) { return reinterpret_cast<float4*>(p); };
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += stride) {
+    const float4 x = rows(b.X)[i];
+    if (copy_best) rows(b.Xbest)[i] = x;
+    if (done) continue;
+    const bool p_in = !init_mode && use_p;
+    const float4 ax = rows(b.AX)[i];
+    const float4 r = init_mode ? zero : rows(b.R)[i], ar = init_mode ? zero : rows(b.AR)[i];
+    const float4 p = p_in ? rows(b.P)[i] : zero, ap = p_in ? rows(b.AP)[i] : zero;
+    double pn[4] = {0.0, 0.0, 0.0, 0.0}, apn[4] = {0.0, 0.0, 0.0, 0.0};
+    // v C_w and av C_w added to the two products
+    auto add = [&](const float4& v, const float4& av, int w) {
+      const float s[4] = {v.x, v.y, v.z, v.w}, t[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const double2 k0 = *reinterpret_cast<const double2*>(&sC[w][c][0]);
+        const double2 k1 = *reinterpret_cast<const double2*>(&sC[w][c][2]);
+        const double k[4] = {k0.x, k0.y, k1.x, k1.y};
+        const double sc = static_cast<double>(s[c]), tc = static_cast<double>(t[c]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          pn[j] = fma(sc, k[j], pn[j]);
+          apn[j] = fma(tc, k[j], apn[j]);
+        }
+      }
+    };
+    auto out = [&](const double (&v)[4]) {
+      return make_float4(static_cast<float>(v[0]), m > 1 ? static_cast<float>(v[1]) : 0.f,
+                         m > 2 ? static_cast<float>(v[2]) : 0.f, m > 3 ? static_cast<float>(v[3]) : 0.f);
+    };
+    if (!init_mode) {
+      add(r, ar, 1);
+      if (use_p) add(p, ap, 2);
+      rows(b.P)[i] = out(pn);
+      rows(b.AP)[i] = out(apn);
+    }
+    add(x, ax, 0);
+    const float4 xo = out(pn), axo = out(apn);
+    auto res = [&](float a, float v, int j) {
+      return j < m ? static_cast<float>(static_cast<double>(a) - sLam[j] * static_cast<double>(v)) : 0.f;
+    };
+    rows(b.X)[i] = xo;
+    rows(b.AX)[i] = axo;
+    rows(b.R)[i] = make_float4(res(axo.x, xo.x, 0), res(axo.y, xo.y, 1), res(axo.z, xo.z, 2), res(axo.w, xo.w, 3));
   }
 }
 
@@ -1364,20 +1387,12 @@ void gram_dev(const Exec& ex, GramWork& w, GramMode mode, const XT* const* blk, 
     return;
   }
   if ((iter || xonly) && m == 4 && ld == 4 && !gram4_old_forced()) {
-    // 4-column blocks: the task-split kernel
-    static std::atomic<int> resident_t[2][64];
-    const int ti = sizeof(XT) == 8 ? 1 : 0;
-    SI_REQUIRE(ex.device >= 0 && ex.device < 64, SI_INVALID_ARGUMENT, "gram: device ordinal");
-    if (resident_t[ti][ex.device] == 0) {
-      int r = 0;
-      SI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_gram4t<XT>, GT_THREADS, 0));
-      resident_t[ti][ex.device] = std::max(1, r);
-    }
-    const int64_t ntiles = (n + GT_TR - 1) / GT_TR;
-    const int grid = static_cast<int>(
-        std::max<int64_t>(1, std::min<int64_t>(ntiles, int64_t(ex.sms) * resident_t[ti][ex.device].load())));
+    // 4-column blocks: the matrix-instruction kernel, two CTAs an SM
+    constexpr int per = GM_THREADS / 32 * GM_UNROLL;
+    const int64_t need = ((n + 3) / 4 + per - 1) / per;
+    const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(ex.sms) * 2)));
     w.ensure(static_cast<size_t>(grid) * 288, ex.stream);
-    k_gram4t<XT><<<grid, GT_THREADS, 0, ex.stream>>>(six[0], six[1], six[2], six[3], six[4], six[5], n,
+    k_gram4m<XT><<<grid, GM_THREADS, 0, ex.stream>>>(six[0], six[1], six[2], six[3], six[4], six[5], n,
                                                      w.partial.get(), stop);
     SI_LAUNCH_CHECK();
     k_gram4_reduce<<<9, 256, 0, ex.stream>>>(w.partial.get(), grid, ns_out, out, stop);
@@ -1547,9 +1562,12 @@ void lobpcg_update_dev(const Exec& ex, const LobpcgBlocks<XT>& b, const LobpcgCt
                        int init_mode) {
   if (n == 0) return;
   const int grid = grid_rows(ex, n);
-  if (ld == 4)
-    k_lobpcg_update4<XT><<<grid_rows(ex, n * 4), 256, 0, ex.stream>>>(b, ctrl, n, init_mode);
-  else if (ld == 8)
+  if (ld == 4) {
+    if constexpr (sizeof(XT) == 4)
+      k_lobpcg_update4_f32<<<grid, 256, 0, ex.stream>>>(b, ctrl, n, init_mode);
+    else
+      k_lobpcg_update4<XT><<<grid_rows(ex, n * 4), 256, 0, ex.stream>>>(b, ctrl, n, init_mode);
+  } else if (ld == 8)
     k_lobpcg_update_q<XT, 8><<<grid_rows(ex, n * 2), 256, 0, ex.stream>>>(b, ctrl, n, init_mode);
   else if (ld == 16)
     k_lobpcg_update_q<XT, 16><<<grid_rows(ex, n * 4), 256, 0, ex.stream>>>(b, ctrl, n, init_mode);
