@@ -3,6 +3,7 @@
 // message for si_last_error(); nothing unwinds across the ABI.
 #include <cuda_runtime.h>
 
+#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -411,8 +412,7 @@ si_status si_spmm(si_ctx* ctx, const si_operator* op, const double* x, double* y
     si::OpDev o = op_of(op);
     SI_REQUIRE(k >= 1, SI_INVALID_ARGUMENT, "k must be >= 1");
     si::RowBlocks rb;
-    si::make_row_blocks(ex, o, rb);
-    rb.attach(o);
+    si::attach_ruled(ex, o, rb, false);
     si::Epilogue<double> ep;
     si::spmm_dev<double>(ex, o, x, y, static_cast<int>(k), static_cast<int>(k), ep);
     SI_CUDA(cudaStreamSynchronize(ex.stream));
@@ -425,8 +425,7 @@ si_status si_spmm_f32(si_ctx* ctx, const si_operator* op, const float* x, float*
     si::OpDev o = op_of(op);
     SI_REQUIRE(k >= 1, SI_INVALID_ARGUMENT, "k must be >= 1");
     si::RowBlocks rb;
-    si::make_row_blocks(ex, o, rb);
-    rb.attach(o);
+    si::attach_ruled(ex, o, rb, false);
     si::Epilogue<float> ep;
     si::spmm_dev<float>(ex, o, x, y, static_cast<int>(k), static_cast<int>(k), ep, nullptr, true);
     SI_CUDA(cudaStreamSynchronize(ex.stream));
@@ -447,9 +446,15 @@ si_status si_operator_plan_create(si_ctx* ctx, const si_operator* op, si_operato
     std::unique_ptr<si_operator_plan> p(new si_operator_plan());
     p->device = ctx->device;
     p->op = op_of(op);
-    si::make_row_blocks(ex, p->op, p->rb);
-    p->rb.sell_ok = true;
-    p->rb.attach(p->op);
+    p->rb.sell_budget = si::free_memory_quarter();
+    if (std::getenv("SPECTRAL_INIT_SPMM_TUNE_FILE") != nullptr) {  // kernels by timing, kept in that file
+      si::make_row_blocks(ex, p->op, p->rb);
+      p->rb.sell_ok = true;
+      p->rb.attach(p->op);
+    } else {
+      si::attach_ruled(ex, p->op, p->rb, true);
+      si::build_sliced_copy(ex, p->op);
+    }
     SI_CUDA(cudaStreamSynchronize(ex.stream));
     *out = p.release();
   });

@@ -102,6 +102,10 @@ struct RowBlocks {
   bool sell_ok = false;
   mutable std::unique_ptr<SellLayout> sell;
   mutable bool sell_failed = false;
+  uint64_t sell_budget = 0;  // most bytes the copy may take (0: not asked for)
+  // kernels by the rule on shape and types instead of by timing candidates
+  // (operators of one solve or one call, whose first pass is what counts)
+  bool ruled = false;
   void attach(OpDev& op) const {
     op.row_blocks = starts.get();
     op.block_ptr = ptrs.get();
@@ -113,6 +117,12 @@ struct RowBlocks {
   }
 };
 void make_row_blocks(const Exec& ex, const OpDev& op, RowBlocks& rb);
+// An operator of one solve (sell_ok: applied many times) or one call: kernels
+// by rule, the partitions above only when a forced kernel may need them.
+void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok);
+uint64_t free_memory_quarter();
+// Build the sliced copy of an attached operator now, where the rule uses it.
+void build_sliced_copy(const Exec& ex, const OpDev& op);
 
 // Epilogue of an SpMM: out = alpha * (A x) + beta * z1 + gamma * z2 + delta * z3
 // (z pointers share the layout of y; a null z contributes nothing).
@@ -156,7 +166,7 @@ template <class XT>
 void spmm_dev(const Exec& ex, const OpDev& op, const XT* x, XT* y, int ld, int k, const Epilogue<XT>& ep,
               const int* stop = nullptr, bool use_f32_values = false);
 // Rows per group chosen for the operator's degree profile.
-int spmm_group_lanes(const OpDev& op);
+int spmm_group_lanes(const OpDev& op, int ld);
 
 // ---- block_ops.cu -----------------------------------------------------------
 constexpr int MAXM = 16;   // widest LOBPCG block

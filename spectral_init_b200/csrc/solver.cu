@@ -45,6 +45,28 @@ constexpr int64_t DENSE_MAX_N = 8192;  // largest n the device dense EVD accepts
 
 namespace {
 
+// Runs a solve on the operator with a sliced copy of its own (built when a
+// kernel first wants it; the caller's where it brings one).  The copy is not
+// worth a solve: one that runs out of memory beside it starts over without.
+template <class F>
+auto with_copy(const Exec& ex, const OpDev& op_in, SolverStats& st, F&& solve) {
+  OpDev op = op_in;
+  RowBlocks rb;
+  if (op.panels != nullptr || op.n <= 0) return solve(op);
+  attach_ruled(ex, op, rb, true);
+  const SolverStats before = st;
+  try {
+    return solve(op);
+  } catch (const Error& e) {
+    if (e.code != SI_OUT_OF_MEMORY || !rb.sell) throw;
+  }
+  cudaGetLastError();  // the failed allocation's
+  rb.sell.reset();
+  rb.sell_failed = true;
+  st = before;
+  return solve(op);
+}
+
 int pick_ld(int m) { return m <= 4 ? 4 : (m <= 8 ? 8 : 16); }
 
 // Block width: the wanted k vectors plus guard vectors up to the padded row
@@ -341,16 +363,18 @@ double max_eigenpair_residual_dev(const Exec& ex, const OpDev& op, const EigenRe
   return acc;
 }
 
+static bool lobpcg_solve_on(const Exec& ex, const OpDev& op, int n_components, uint64_t seed, bool regularize,
+                            const double* sqrt_deg, const SolverConfig& cfg, EigenResult& out, SolverStats& st);
+
 bool lobpcg_solve_dev(const Exec& ex, const OpDev& op_in, int n_components, uint64_t seed, bool regularize,
                       const double* sqrt_deg, const SolverConfig& cfg, EigenResult& out, SolverStats& st) {
-  // row partition for the tiled SpMM (built once per solve when absent)
-  RowBlocks row_blocks_;
-  OpDev op = op_in;
-  if (op.row_blocks == nullptr && op.n > 0) {
-    make_row_blocks(ex, op, row_blocks_);
-    row_blocks_.sell_ok = true;
-    row_blocks_.attach(op);
-  }
+  return with_copy(ex, op_in, st, [&](const OpDev& op) {
+    return lobpcg_solve_on(ex, op, n_components, seed, regularize, sqrt_deg, cfg, out, st);
+  });
+}
+
+static bool lobpcg_solve_on(const Exec& ex, const OpDev& op, int n_components, uint64_t seed, bool regularize,
+                     const double* sqrt_deg, const SolverConfig& cfg, EigenResult& out, SolverStats& st) {
   const int64_t n = op.n;
   const int k = n_components + 1;
   if (n_components <= 0 || k >= n) return false;
@@ -500,15 +524,8 @@ bool lobpcg_solve_dev(const Exec& ex, const OpDev& op_in, int n_components, uint
 // ascending order.  The crate applies M^-1 through a sparse Cholesky factor;
 // here each application is a block CG solve on the same CSR SpMM (relative
 // residual 1e-12), so the factorisation is never formed.
-bool sinv_solve_dev(const Exec& ex, const OpDev& op_in, int n_components, uint64_t seed, const double* sqrt_deg,
+bool sinv_solve_dev(const Exec& ex, const OpDev& op, int n_components, uint64_t seed, const double* sqrt_deg,
                     const SolverConfig& cfg, EigenResult& out, SolverStats& st) {
-  RowBlocks row_blocks_;
-  OpDev op = op_in;
-  if (op.row_blocks == nullptr && op.n > 0) {
-    make_row_blocks(ex, op, row_blocks_);
-    row_blocks_.sell_ok = true;
-    row_blocks_.attach(op);
-  }
   const int64_t n = op.n;
   const int k = n_components + 1;
   if (n_components <= 0 || k >= n || sqrt_deg == nullptr) return false;
@@ -633,16 +650,18 @@ int rsvd_width(int64_t n, int n_components, int oversampling) {
   return oversampling < 0 ? rsvd_k_sub(n, rank) : static_cast<int>(std::min<int64_t>(rank + oversampling, n));
 }
 
+static void rsvd_solve_on(const Exec& ex, const OpDev& op, int n_components, uint64_t seed, int oversampling,
+                          int nbiter, EigenResult& out, SolverStats& st);
+
 void rsvd_solve_dev(const Exec& ex, const OpDev& op_in, int n_components, uint64_t seed, int oversampling, int nbiter,
                     EigenResult& out, SolverStats& st) {
-  // row partition for the tiled SpMM (built once per solve when absent)
-  RowBlocks row_blocks_;
-  OpDev op = op_in;
-  if (op.row_blocks == nullptr && op.n > 0) {
-    make_row_blocks(ex, op, row_blocks_);
-    row_blocks_.sell_ok = true;
-    row_blocks_.attach(op);
-  }
+  with_copy(ex, op_in, st, [&](const OpDev& op) {
+    rsvd_solve_on(ex, op, n_components, seed, oversampling, nbiter, out, st);
+  });
+}
+
+static void rsvd_solve_on(const Exec& ex, const OpDev& op, int n_components, uint64_t seed, int oversampling,
+                          int nbiter, EigenResult& out, SolverStats& st) {
   const int64_t n = op.n;
   SI_REQUIRE(n_components > 0 && n_components < n, SI_INVALID_ARGUMENT, "rsvd: need 0 < n_components < n");
   const int rank = n_components + 1;
@@ -711,16 +730,18 @@ void dense_evd_result(const Exec& ex, const OpDev& op, int k, EigenResult& out) 
   dense_evd_dev(ex, op, k, out.vals.data(), out.vecs.get(), k);
 }
 
+static void solve_chain_on(const Exec& ex, const OpDev& op, int n_components, uint64_t seed, const double* sqrt_deg,
+                           const SolverConfig& cfg, EigenResult& out, SolverStats& st);
+
 void solve_eigenproblem_dev(const Exec& ex, const OpDev& op_in, int n_components, uint64_t seed, const double* sqrt_deg,
                             const SolverConfig& cfg, EigenResult& out, SolverStats& st) {
-  // row partition for the tiled SpMM (built once per solve when absent)
-  RowBlocks row_blocks_;
-  OpDev op = op_in;
-  if (op.row_blocks == nullptr && op.n > 0) {
-    make_row_blocks(ex, op, row_blocks_);
-    row_blocks_.sell_ok = true;
-    row_blocks_.attach(op);
-  }
+  with_copy(ex, op_in, st, [&](const OpDev& op) {
+    solve_chain_on(ex, op, n_components, seed, sqrt_deg, cfg, out, st);
+  });
+}
+
+static void solve_chain_on(const Exec& ex, const OpDev& op, int n_components, uint64_t seed, const double* sqrt_deg,
+                           const SolverConfig& cfg, EigenResult& out, SolverStats& st) {
   const int64_t n = op.n;
   const int k = n_components + 1;
   const int fl = cfg.force_level;

@@ -1074,12 +1074,27 @@ __global__ void k_sell_fill(int64_t n_slices, const uint64_t* __restrict__ slice
     const uint32_t row = perm[s * 32 + lane];
     const uint64_t len = plen[s * 32 + lane];
     const uint64_t src = row != 0xffffffffu ? indptr[row] : 0;
-    for (uint64_t j = 0; j < w; ++j) {
-      const uint64_t slot = base + 32 * j + lane;
-      const bool ok = j < len;
-      sidx[slot] = ok ? indices[src + j] : 0u;
-      if (s32 != nullptr) s32[slot] = ok ? v32[src + j] : 0.0f;
-      if (s64 != nullptr) s64[slot] = ok ? v64[src + j] : 0.0;
+    // four positions' loads in flight: a lane walks its own row, so a request
+    // touches up to 32 lines and only its latency bounds the copy
+    for (uint64_t j0 = 0; j0 < w; j0 += 4) {
+      uint32_t c[4];
+      float f[4];
+      double g[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool ok = j0 + u < len;
+        c[u] = ok ? indices[src + j0 + u] : 0u;
+        f[u] = ok && s32 != nullptr ? v32[src + j0 + u] : 0.0f;
+        g[u] = ok && s64 != nullptr ? v64[src + j0 + u] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (j0 + u >= w) break;
+        const uint64_t slot = base + 32 * (j0 + u) + lane;
+        sidx[slot] = c[u];
+        if (s32 != nullptr) s32[slot] = f[u];
+        if (s64 != nullptr) s64[slot] = g[u];
+      }
     }
   }
 }
@@ -1278,6 +1293,16 @@ __global__ void __launch_bounds__(NT, 1) k_spmm_sell(SellArgs a, const VT* __res
   }
 }
 
+}  // namespace
+
+uint64_t free_memory_quarter() {
+  size_t free_b = 0, total_b = 0;
+  SI_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  return std::max<uint64_t>(free_b / 4, 1);
+}
+
+namespace {
+
 // The sliced-ELL copy of the operator (built on first use, outside stream
 // capture, for owners that allow it; null when not available).
 const SellLayout* sell_layout(const Exec& ex, const OpDev& op) {
@@ -1316,12 +1341,15 @@ const SellLayout* sell_layout(const Exec& ex, const OpDev& op) {
   SI_LAUNCH_CHECK();
   L->slice_ptr.alloc(static_cast<size_t>(L->n_slices + 1), ex.stream);
   L->slots = exclusive_scan_u64(ex, cnt.get(), L->slice_ptr.get(), L->n_slices);
-  // the copy must fit beside the solver's work buffers: at most a quarter of
-  // the free memory
+  // The copy must fit beside what else the program needs: a prepared operator
+  // has its budget from its creation; a solve, which drops the copy again when
+  // it runs out of memory, asks the driver only for copies of gigabytes
+  // (cudaMemGetInfo was seen to take 30 to 80 ms behind queued frees).
   const size_t per_slot = 4 + (op.v32 ? 4 : 0) + (op.v64 ? 8 : 0);
-  size_t free_b = 0, total_b = 0;
-  SI_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  if (L->slots * per_slot > free_b / 4) {
+  const uint64_t want = L->slots * per_slot;
+  uint64_t budget = op.panels->sell_budget;
+  if (budget == 0 && want > uint64_t(2) << 30) budget = free_memory_quarter();
+  if (budget != 0 && want > budget) {
     op.panels->sell_failed = true;
     return nullptr;
   }
@@ -1384,7 +1412,7 @@ void launch_lanes(int g, const Exec& ex, const OpDev& op, const VT* vals, const 
                   const int* stop) {
   if (g == 300) {
     if (launch_panel<VT, XT, LD>(ex, op, vals, x, y, ep, stop)) return;
-    g = spmm_group_lanes(op);  // no windows (inside a capture before first use): direct kernel
+    g = spmm_group_lanes(op, LD);  // no windows (inside a capture before first use): direct kernel
   }
   if (g >= 400 && g <= 403) {
     bool ok = false;
@@ -1395,7 +1423,7 @@ void launch_lanes(int g, const Exec& ex, const OpDev& op, const VT* vals, const 
       default: ok = launch_sell<VT, XT, LD, true, true, true>(ex, op, vals, x, y, ep, stop); break;
     }
     if (ok) return;
-    g = spmm_group_lanes(op);  // no sliced copy: direct kernel
+    g = spmm_group_lanes(op, LD);  // no sliced copy: direct kernel
   }
   switch (g) {
     case 4: launch_vec<VT, XT, LD, 4>(ex, op, vals, x, y, ep, stop); break;
@@ -1506,6 +1534,58 @@ int forced_choice(const OpDev& op, bool tiled) {
   return 0;
 }
 
+// Kernel by shape and types.  Timing candidates would cost an operator's first
+// pass more than it gains (13 candidates: 36 ms of a 77 ms first solve at n =
+// 1M, 4.9 ms before a product of 90 us at n = 300k); operators prepared with a
+// tuning file still do.  The sliced kernels, where the operator allows its
+// copy, from the size at which they beat the best CSR vector kernel (us, sliced
+// against vector; f64, 4 columns: 27 / 24 with 1.4 M entries, 54 / 75 with 4.9
+// M, 160 / 219 with 24 M; f32 alike), with the next slice prefetched while x
+// is small (57 / 54 without / with at n = 100k, 160 / 168 at n = 1M).  Wider
+// rows gain from them only once the block outgrows the L2's reach (8 columns,
+// f64: 84 / 84 with 4.9 M, 312 / 354 at n = 1M; 16 columns, f32: 140 / 113 and
+// 480 / 541), and 16 f64 columns gain nothing clear (780 / 710 in cluster order,
+// 805 / 827 shuffled; four passes of four columns: 1051 and 1182).
+template <class VT, class XT, int LD>
+int ruled_choice(const OpDev& op) {
+  const bool large = op.n >= int64_t(1) << 19;
+  if (op.panels->sell_ok && op.nnz >= kTuneMinNnz) {
+    if (LD == 4) return large ? 402 : 403;
+    if (large) {
+      if (std::is_same<XT, float>::value) return 403;
+      if (LD == 8) return 401;
+    }
+  }
+  return spmm_group_lanes(op, LD);
+}
+
+// Blocks whose row stride or alignment the vector gathers cannot take: packed
+// into an aligned block of 4, 8 or 16 columns and the product unpacked.
+template <class XT>
+__global__ void k_pad_rows(int64_t n, int k, const XT* __restrict__ in, int ld_in, XT* __restrict__ out, int ld_out) {
+  const int64_t total = n * ld_out;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total; e += stride) {
+    const int64_t i = e / ld_out;
+    const int c = static_cast<int>(e - i * ld_out);
+    out[e] = c < k ? in[i * ld_in + c] : XT(0);
+  }
+}
+
+template <class XT>
+__global__ void k_unpad_rows(int64_t n, int k, const XT* __restrict__ in, int ld_in, XT* __restrict__ out,
+                             int ld_out) {
+  const int64_t total = n * k;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total; e += stride) {
+    const int64_t i = e / k;
+    const int c = static_cast<int>(e - i * k);
+    out[i * ld_out + c] = in[i * ld_in + c];
+  }
+}
+
+constexpr int64_t kPadMinNnz = int64_t(3) << 17;
+
 template <class VT, class XT, int LD>
 void dispatch_g(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* y, const Epilogue<XT>& ep,
                 const int* stop) {
@@ -1515,6 +1595,7 @@ void dispatch_g(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT
   const TuneKey key{ex.device, op.indptr, op.indices, op.n, op.nnz, LD, static_cast<int>(sizeof(VT)),
                     static_cast<int>(sizeof(XT)), tiled ? 1 : 0, panel ? 1 : 0, sell ? 1 : 0};
   int g = forced_choice<VT, XT, LD>(op, tiled);
+  if (g == 0 && op.panels != nullptr && op.panels->ruled) g = ruled_choice<VT, XT, LD>(op);
   if (g != 0) {
     launch_lanes<VT, XT, LD>(g, ex, op, vals, x, y, ep, stop);
     return;
@@ -1538,15 +1619,9 @@ void dispatch_g(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     SI_CUDA(cudaStreamIsCapturing(ex.stream, &cs));
     // below ~4 M stored entries timing the candidates (and building the
-    // sliced copy for them) costs more than a better kernel saves over a solve:
-    // measured on 502 components of 20 to 100 k nodes, the CSR vector kernel
-    // alone finished the workload in 1.17 s, the tuned run in 1.20 / 1.44 s
-    const bool tiny = op.n < 20000;
-    const bool small = op.nnz < kTuneMinNnz;
-    if (cs != cudaStreamCaptureStatusNone || tiny) {
-      g = tiled ? 104 : spmm_group_lanes(op);
-    } else if (small) {
-      g = spmm_group_lanes(op);
+    // sliced copy for them) costs more than a better kernel saves
+    if (cs != cudaStreamCaptureStatusNone || op.nnz < kTuneMinNnz) {
+      g = spmm_group_lanes(op, LD);
     } else {
       timed = true;
       cudaEvent_t e0, e1;
@@ -1599,7 +1674,25 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
   if (aligned && ld == 4) return dispatch_g<VT, XT, 4>(ex, op, vals, x, y, ep, stop);
   if (aligned && ld == 8) return dispatch_g<VT, XT, 8>(ex, op, vals, x, y, ep, stop);
   if (aligned && ld == 16) return dispatch_g<VT, XT, 16>(ex, op, vals, x, y, ep, stop);
-  switch (spmm_group_lanes(op)) {
+  if (k <= 16 && op.nnz >= kPadMinNnz && ep.z1 == nullptr && ep.z2 == nullptr && ep.z3 == nullptr && stop == nullptr) {
+    // the scalar gathers of the generic kernel cost a request per column and
+    // entry (us, generic against this, f64: 1 column 113 / 84 and 3 columns 129 /
+    // 86 at n = 300k shuffled, 9 columns 774 / 588 at n = 800k; level at n = 20k)
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    SI_CUDA(cudaStreamIsCapturing(ex.stream, &cs));
+    if (cs == cudaStreamCaptureStatusNone) {
+      const int lp = k <= 4 ? 4 : (k <= 8 ? 8 : 16);
+      DevBuf<XT> xp(static_cast<size_t>(op.n) * lp, ex.stream), yp(static_cast<size_t>(op.n) * lp, ex.stream);
+      const int g1 = static_cast<int>(std::min<int64_t>((op.n * lp + 255) / 256, int64_t(ex.sms) * 16));
+      k_pad_rows<XT><<<g1, 256, 0, ex.stream>>>(op.n, k, x, ld, xp.get(), lp);
+      SI_LAUNCH_CHECK();
+      dispatch<VT, XT>(ex, op, vals, xp.get(), yp.get(), lp, k, ep, stop);
+      k_unpad_rows<XT><<<g1, 256, 0, ex.stream>>>(op.n, k, yp.get(), lp, y, ld);
+      SI_LAUNCH_CHECK();
+      return;
+    }
+  }
+  switch (spmm_group_lanes(op, 4)) {
     case 4: return launch_generic<VT, XT, 4>(ex, op, vals, x, y, ld, k, ep, stop);
     case 8: return launch_generic<VT, XT, 8>(ex, op, vals, x, y, ld, k, ep, stop);
     case 16: return launch_generic<VT, XT, 16>(ex, op, vals, x, y, ld, k, ep, stop);
@@ -1608,6 +1701,23 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
 }
 
 }  // namespace
+
+void build_sliced_copy(const Exec& ex, const OpDev& op) {
+  if (op.nnz >= kTuneMinNnz) sell_layout(ex, op);
+}
+
+void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok) {
+  for (const char* name :
+       {"SPECTRAL_INIT_SPMM_KERNEL", "SPECTRAL_INIT_SPMM_KERNEL_F32", "SPECTRAL_INIT_SPMM_KERNEL_F64"}) {
+    if (std::getenv(name) != nullptr) {
+      make_row_blocks(ex, op, rb);
+      break;
+    }
+  }
+  rb.sell_ok = sell_ok;
+  rb.ruled = true;
+  rb.attach(op);
+}
 
 void make_row_blocks(const Exec& ex, const OpDev& op, RowBlocks& rb) {
   auto build = [&](int64_t per, int64_t& nb, DevBuf<int64_t>& starts, DevBuf<uint64_t>& ptrs) {
@@ -1628,14 +1738,19 @@ void make_row_blocks(const Exec& ex, const OpDev& op, RowBlocks& rb) {
   rb.sell_failed = false;
 }
 
-int spmm_group_lanes(const OpDev& op) {
-  // a lane covers up to 8 entries per pass: fewest lanes that keep most rows
-  // to one pass (more rows in flight per SM beats wider groups)
+int spmm_group_lanes(const OpDev& op, int ld) {
+  // A lane covers up to 8 entries per pass: the fewest lanes that keep most
+  // rows to one pass, since more rows in flight per SM beats wider groups --
+  // as long as there are rows enough to fill the GPU.  Below half a million
+  // lanes wider groups win (f64, 4 columns, us with 4 / 8 / 16 / 32 lanes: 31 /
+  // 29 / 18 / 15 at n = 20 000, 31 / 31 / 24 / 27 at 60 000, 77 / 78 / 71 / 89
+  // at 200 000); 8 and 16 columns leave a lane enough columns to reduce only
+  // from 16 lanes on (16 columns at n = 60 000: 82 / 74 / 57 / 64).
   const double mean = op.n > 0 ? static_cast<double>(op.nnz) / static_cast<double>(op.n) : 0.0;
-  if (mean <= 28.0) return 4;
-  if (mean <= 56.0) return 8;
-  if (mean <= 112.0) return 16;
-  return 32;
+  int g = mean <= 28.0 ? 4 : (mean <= 56.0 ? 8 : (mean <= 112.0 ? 16 : 32));
+  if (ld >= 8) g = std::max(g, 16);
+  while (g < 32 && op.n * g < int64_t(1) << 19) g *= 2;
+  return g;
 }
 
 template <class XT>
