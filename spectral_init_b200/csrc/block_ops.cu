@@ -270,11 +270,12 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 }
 
 template <class XT>
-__global__ void __launch_bounds__(GM_THREADS) k_gram4m(const XT* __restrict__ X, const XT* __restrict__ R,
-                                                       const XT* __restrict__ P, const XT* __restrict__ AX,
-                                                       const XT* __restrict__ AR, const XT* __restrict__ AP,
-                                                       int64_t n, double* __restrict__ partial,
-                                                       const int* __restrict__ stop) {
+__global__ void __launch_bounds__(GM_THREADS) k_gram4m(const XT* X, const XT* R,
+                                                       const XT* P, const XT* AX,
+                                                       const XT* AR, const XT* AP,
+                                                       int64_t n, double* partial,
+                                                       const int* stop) {
+  kernel_begin();
   if (stop != nullptr && *stop != 0) return;
   constexpr int NW = GM_THREADS / 32;
   __shared__ double red[NW][4][64];
@@ -352,8 +353,9 @@ bool gram4_old_forced() {
 // w + 8, ..., then the warp sums in warp order) and writes both
 // (4 ns_out) x (4 ns_out) matrices (upper triangles mirrored); ns_out = 1
 // keeps only the first block of S and of AS (the Gram of X and AX alone).
-__global__ void __launch_bounds__(256) k_gram4_reduce(const double* __restrict__ partial, int nparts, int ns_out,
-                                                      double* __restrict__ out, const int* __restrict__ stop) {
+__global__ void __launch_bounds__(256) k_gram4_reduce(const double* partial, int nparts, int ns_out,
+                                                      double* out, const int* stop) {
+  kernel_begin();
   if (stop != nullptr && *stop != 0) return;
   __shared__ double red[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -423,11 +425,12 @@ __device__ __forceinline__ void upper_tile(int u, int& ti, int& tj) {
 
 template <class XT, int LD>
 __global__ void __maxnreg__(128)
-    k_gram_ld(const XT* __restrict__ X, const XT* __restrict__ R, const XT* __restrict__ P,
-              const XT* __restrict__ AX, const XT* __restrict__ AR, const XT* __restrict__ AP, int64_t n,
-              double* __restrict__ partial, const int* __restrict__ stop) {
+    k_gram_ld(const XT* X, const XT* R, const XT* P,
+              const XT* AX, const XT* AR, const XT* AP, int64_t n,
+              double* partial, const int* stop) {
   using C = GramLd<LD>;
   constexpr int TS = C::TS, SW = gram_ld_stride<XT, LD>();
+  kernel_begin();
   if (stop != nullptr && *stop != 0) return;
   extern __shared__ __align__(16) unsigned char gram_ld_raw[];
   XT* tile = reinterpret_cast<XT*>(gram_ld_raw);
@@ -523,11 +526,12 @@ __global__ void __maxnreg__(128)
 // (3m) x (3m) matrices.  A CTA takes 32 entries: warp w adds CTAs w, w + 8,
 // ..., then the eight warp sums are added in warp order.
 template <int LD>
-__global__ void __launch_bounds__(256) k_gram_ld_reduce(const double* __restrict__ partial, int nparts, int m,
-                                                        int ns_out, double* __restrict__ out,
-                                                        const int* __restrict__ stop) {
+__global__ void __launch_bounds__(256) k_gram_ld_reduce(const double* partial, int nparts, int m,
+                                                        int ns_out, double* out,
+                                                        const int* stop) {
   using C = GramLd<LD>;
   constexpr int TS = C::TS;
+  kernel_begin();
   if (stop != nullptr && *stop != 0) return;
   __shared__ double red[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -560,11 +564,12 @@ __global__ void __launch_bounds__(256) k_gram_ld_reduce(const double* __restrict
 // output column j (inputs are read as 4-vectors; the four threads of a row
 // share the same sectors).
 template <class XT>
-__global__ void __launch_bounds__(256) k_lobpcg_update4(LobpcgBlocks<XT> b, const LobpcgCtrl* __restrict__ ctrl,
+__global__ void __launch_bounds__(256) k_lobpcg_update4(LobpcgBlocks<XT> b, const LobpcgCtrl* ctrl,
                                                         int64_t n, int init_mode) {
   __shared__ double sC[3][4][4];
   __shared__ double sLam[4];
   __shared__ int sF[4];
+  kernel_begin();
   if (threadIdx.x == 0) {
     sF[0] = ctrl->done;
     sF[1] = ctrl->copy_best;
@@ -640,11 +645,12 @@ __global__ void __launch_bounds__(256) k_lobpcg_update4(LobpcgBlocks<XT> b, cons
 // converted to f64 once (four threads a row each convert the row: 116
 // conversions a row, and the unit does 16 a clock and SM, against 52 here).
 // n = 1M: 54 -> 36 us, floor 27 us (11 n ld s bytes).
-__global__ void __launch_bounds__(256, 2) k_lobpcg_update4_f32(LobpcgBlocks<float> b, const LobpcgCtrl* __restrict__ ctrl,
+__global__ void __launch_bounds__(256, 2) k_lobpcg_update4_f32(LobpcgBlocks<float> b, const LobpcgCtrl* ctrl,
                                                             int64_t n, int init_mode) {
   __shared__ __align__(16) double sC[3][4][4];  // [block][input column][output column]
   __shared__ double sLam[4];
   __shared__ int sF[4];
+  kernel_begin();
   if (threadIdx.x == 0) {
     sF[0] = ctrl->done;
     sF[1] = ctrl->copy_best;
@@ -1157,13 +1163,14 @@ struct Vec16<float> {
 // from shared memory (zero outside the m x m block).  Same formulas as
 // k_lobpcg_update.
 template <class XT, int LD>
-__global__ void __launch_bounds__(256) k_lobpcg_update_q(LobpcgBlocks<XT> b, const LobpcgCtrl* __restrict__ ctrl,
+__global__ void __launch_bounds__(256) k_lobpcg_update_q(LobpcgBlocks<XT> b, const LobpcgCtrl* ctrl,
                                                          int64_t n, int init_mode) {
   constexpr int TPR = LD / 4;
   constexpr int EPV = 16 / sizeof(XT);  // elements per 16-byte load
   using V = typename Vec16<XT>::type;
   __shared__ __align__(16) double sC[3][LD][LD];
   __shared__ double sLam[LD];
+  kernel_begin();
   const int done = ctrl->done, copy_best = ctrl->copy_best, use_p = ctrl->has_p, m = ctrl->m;
   if (done && !copy_best) return;
   for (int i = threadIdx.x; i < 3 * LD * LD; i += blockDim.x) {
@@ -1358,10 +1365,11 @@ void gram_ld_launch(const Exec& ex, GramWork& w, const XT* const* blk, int m, in
   const int grid = static_cast<int>(
       std::max<int64_t>(1, std::min<int64_t>(ntiles, int64_t(ex.sms) * resident[ex.device].load())));
   w.ensure(static_cast<size_t>(grid) * C::ENTRIES, ex.stream);
-  k_gram_ld<XT, LD><<<grid, C::THREADS, smem, ex.stream>>>(blk[0], blk[1], blk[2], blk[3], blk[4], blk[5], n,
-                                                           w.partial.get(), stop);
+  launch_after(ex.stream, k_gram_ld<XT, LD>, grid, C::THREADS, smem, blk[0], blk[1], blk[2], blk[3], blk[4], blk[5], n,
+               w.partial.get(), stop);
   SI_LAUNCH_CHECK();
-  k_gram_ld_reduce<LD><<<(C::ENTRIES + 31) / 32, 256, 0, ex.stream>>>(w.partial.get(), grid, m, ns_out, out, stop);
+  launch_after(ex.stream, k_gram_ld_reduce<LD>, (C::ENTRIES + 31) / 32, 256, 0,
+               static_cast<const double*>(w.partial.get()), grid, m, ns_out, out, stop);
   SI_LAUNCH_CHECK();
 }
 
@@ -1392,10 +1400,11 @@ void gram_dev(const Exec& ex, GramWork& w, GramMode mode, const XT* const* blk, 
     const int64_t need = ((n + 3) / 4 + per - 1) / per;
     const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(ex.sms) * 2)));
     w.ensure(static_cast<size_t>(grid) * 288, ex.stream);
-    k_gram4m<XT><<<grid, GM_THREADS, 0, ex.stream>>>(six[0], six[1], six[2], six[3], six[4], six[5], n,
-                                                     w.partial.get(), stop);
+    launch_after(ex.stream, k_gram4m<XT>, grid, GM_THREADS, 0, six[0], six[1], six[2], six[3], six[4], six[5], n,
+                 w.partial.get(), stop);
     SI_LAUNCH_CHECK();
-    k_gram4_reduce<<<9, 256, 0, ex.stream>>>(w.partial.get(), grid, ns_out, out, stop);
+    launch_after(ex.stream, k_gram4_reduce, 9, 256, 0, static_cast<const double*>(w.partial.get()), grid, ns_out,
+                 out, stop);
     SI_LAUNCH_CHECK();
     return;
   }
@@ -1564,13 +1573,13 @@ void lobpcg_update_dev(const Exec& ex, const LobpcgBlocks<XT>& b, const LobpcgCt
   const int grid = grid_rows(ex, n);
   if (ld == 4) {
     if constexpr (sizeof(XT) == 4)
-      k_lobpcg_update4_f32<<<grid, 256, 0, ex.stream>>>(b, ctrl, n, init_mode);
+      launch_after(ex.stream, k_lobpcg_update4_f32, grid, 256, 0, b, ctrl, n, init_mode);
     else
-      k_lobpcg_update4<XT><<<grid_rows(ex, n * 4), 256, 0, ex.stream>>>(b, ctrl, n, init_mode);
+      launch_after(ex.stream, k_lobpcg_update4<XT>, grid_rows(ex, n * 4), 256, 0, b, ctrl, n, init_mode);
   } else if (ld == 8)
-    k_lobpcg_update_q<XT, 8><<<grid_rows(ex, n * 2), 256, 0, ex.stream>>>(b, ctrl, n, init_mode);
+    launch_after(ex.stream, k_lobpcg_update_q<XT, 8>, grid_rows(ex, n * 2), 256, 0, b, ctrl, n, init_mode);
   else if (ld == 16)
-    k_lobpcg_update_q<XT, 16><<<grid_rows(ex, n * 4), 256, 0, ex.stream>>>(b, ctrl, n, init_mode);
+    launch_after(ex.stream, k_lobpcg_update_q<XT, 16>, grid_rows(ex, n * 4), 256, 0, b, ctrl, n, init_mode);
   else
     k_lobpcg_update_generic<XT><<<grid, 256, 0, ex.stream>>>(b, ctrl, n, ld, init_mode);
   SI_LAUNCH_CHECK();

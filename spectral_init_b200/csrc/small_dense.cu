@@ -886,13 +886,11 @@ __device__ void warp_householder(double* A, int s, int ld, double* d, double* e,
       s1 = fma(w[k + 1], v[k + 1], s1);
     }
     s0 = fma(w[N - 1], v[N - 1], s0);
-    const double h = 0.5 * tj * tj * (s0 + s1);  // w = tau p - h v
-    const double wown = fma(tj, p, -h * own);
+    // A - v w^T - w v^T with w = tau p - h v, in p: A - v (w - h v)^T - p (tau v)^T
+    const double h = 0.5 * tj * tj * (s0 + s1);
+    const double c1 = fma(tj, p, -2.0 * h * own), c2 = tj * own;
 #pragma unroll
-    for (int k = 1; k < N; ++k) {
-      w[k] = fma(tj, w[k], -h * v[k]);
-      a[k - 1] = on ? a[k] - fma(v[k], wown, w[k] * own) : a[k];
-    }
+    for (int k = 1; k < N; ++k) a[k - 1] = fma(-v[k], c1, fma(-w[k], c2, a[k]));
     a[N - 1] = 0.0;
     if (l > j && l < s) A[j * ld + l] = on ? own : 0.0;
     if (l == 0) {
@@ -1517,7 +1515,7 @@ __device__ bool rr_general(const double* gb, const double* ga, int P, const int*
 // `ctrl` points to the CTA's shared-memory copy of the control block's header;
 // the coefficients, which the step only writes, go to `gctrl` in global memory.
 template <int NT, bool REG, bool PAR>
-__device__ void small_step_body(LobpcgCtrl* ctrl, LobpcgCtrl* gctrl, const double* __restrict__ gram, int ns, int mode,
+__device__ void small_step_body(LobpcgCtrl* ctrl, LobpcgCtrl* gctrl, const double* gram, int ns, int mode,
                                 double* smem) {
   __shared__ double red[ST_WIDE / 32];
   __shared__ double rc[SMAX / 2 + 1], rs[SMAX / 2 + 1], dsc[3 * MAXM], theta[MAXM], rn[MAXM];
@@ -1710,7 +1708,7 @@ __device__ void small_step_body(LobpcgCtrl* ctrl, LobpcgCtrl* gctrl, const doubl
 // (the step is a long chain of small dependent updates) and written back at
 // the end.
 template <int NT, bool REG = false, bool PAR = false>
-__global__ void __launch_bounds__(NT, 1) k_small_step(LobpcgCtrl* ctrl, const double* __restrict__ gram, int ns,
+__global__ void __launch_bounds__(NT, 1) k_small_step(LobpcgCtrl* ctrl, const double* gram, int ns,
                                                    int mode) {
   extern __shared__ double smem[];
   __shared__ LobpcgCtrl sctrl;
@@ -1718,7 +1716,9 @@ __global__ void __launch_bounds__(NT, 1) k_small_step(LobpcgCtrl* ctrl, const do
   static_assert(offsetof(LobpcgCtrl, Cx) % sizeof(double) == 0, "the header must be a whole number of words");
   double* dst = reinterpret_cast<double*>(&sctrl);
   const double* src = reinterpret_cast<const double*>(ctrl);
-  for (int i = threadIdx.x; i < W; i += blockDim.x) dst[i] = src[i];
+  // complete since the previous step (the kernels between have waited for it)
+  for (int i = threadIdx.x; i < W; i += blockDim.x) dst[i] = __ldcg(src + i);
+  kernel_begin();
   __syncthreads();
   small_step_body<NT, REG, PAR>(&sctrl, ctrl, gram, ns, mode, smem);
   __syncthreads();
@@ -1806,16 +1806,20 @@ void small_step_dev(const Exec& ex, LobpcgCtrl* ctrl, const double* gram, int ns
   // one warp)
   const int variant = small_step_variant();
   const bool par = variant != 3;
+  auto launch = [&](auto kernel, int threads) {
+    launch_after(ex.stream, kernel, 1, threads, smem, ctrl, gram, ns, mode);
+  };
   if (ns * m > 24) {
-    if (par) k_small_step<ST_WIDE, false, true><<<1, ST_WIDE, smem, ex.stream>>>(ctrl, gram, ns, mode);
-    else k_small_step<ST_WIDE><<<1, ST_WIDE, smem, ex.stream>>>(ctrl, gram, ns, mode);
+    if (par) launch(k_small_step<ST_WIDE, false, true>, ST_WIDE);
+    else launch(k_small_step<ST_WIDE>, ST_WIDE);
   } else if (ns * m > WRR || variant == 1 || variant == 3) {
-    if (par) k_small_step<ST, false, true><<<1, ST, smem, ex.stream>>>(ctrl, gram, ns, mode);
-    else k_small_step<ST><<<1, ST, smem, ex.stream>>>(ctrl, gram, ns, mode);
-  } else if (variant == 2)
-    k_small_step<32, true><<<1, 32, smem, ex.stream>>>(ctrl, gram, ns, mode);
-  else
-    k_small_step<32><<<1, 32, smem, ex.stream>>>(ctrl, gram, ns, mode);
+    if (par) launch(k_small_step<ST, false, true>, ST);
+    else launch(k_small_step<ST>, ST);
+  } else if (variant == 2) {
+    launch(k_small_step<32, true>, 32);
+  } else {
+    launch(k_small_step<32>, 32);
+  }
   SI_LAUNCH_CHECK();
 }
 

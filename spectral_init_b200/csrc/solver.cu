@@ -312,15 +312,15 @@ void chebyshev_start(const Exec& ex, const OpDev& L, LobpcgState<XT>& s, bool f3
 // Rayleigh-Ritz of the operator on span(src): dst = src V, vals = theta.
 void rr_refine(const Exec& ex, const OpDev& L, LobpcgState<double>& s, const double* src, double* dst,
                std::vector<double>& vals, int& spmm_calls) {
+  LobpcgCtrl h;
+  std::memset(&h, 0, sizeof(h));
+  h.m = s.m;
+  SI_CUDA(cudaMemcpyAsync(s.aux.get(), &h, sizeof(h), cudaMemcpyHostToDevice, ex.stream));
   Epilogue<double> ep;
   spmm_dev<double>(ex, L, src, s.AX.get(), s.ld, s.m, ep);
   ++spmm_calls;
   const double* blk[2] = {src, s.AX.get()};
   gram_dev<double>(ex, s.gw, GRAM_SYM2, blk, 1, 2, s.m, s.ld, s.n, s.gram.get());
-  LobpcgCtrl h;
-  std::memset(&h, 0, sizeof(h));
-  h.m = s.m;
-  SI_CUDA(cudaMemcpyAsync(s.aux.get(), &h, sizeof(h), cudaMemcpyHostToDevice, ex.stream));
   small_step_dev(ex, s.aux.get(), s.gram.get(), 1, SM_RR_PLAIN, s.m);
   const double* in[1] = {src};
   const double* coef[1] = {s.aux.get()->Cx};

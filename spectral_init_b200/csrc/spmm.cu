@@ -81,7 +81,7 @@ struct RowLoadF32x8 {
 #pragma unroll
     for (int q = 0; q < LD / 8; ++q) {
       float a[8];
-      asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                    : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]),
                      "=f"(a[7])
                    : "l"(p + 8 * q));
@@ -229,9 +229,12 @@ template <class VT, class XT, int LD, int G>
 __global__ void __launch_bounds__(256) k_spmm_vec(int64_t n, const uint64_t* __restrict__ indptr,
                                                   const uint32_t* __restrict__ indices,
                                                   const VT* __restrict__ vals, double diag,
-                                                  const XT* __restrict__ x, XT* __restrict__ y,
-                                                  Epilogue<XT> ep, const int* __restrict__ stop) {
+                                                  const XT* x, XT* y,
+                                                  Epilogue<XT> ep, const int* stop) {
+  kernel_begin();
   if (stop != nullptr && *stop != 0) return;
+  x = after_begin(x);
+  indptr = after_begin(indptr);
   const int lane = threadIdx.x & 31;
   const int sub = lane & (G - 1);
   const unsigned mask = group_mask<G>(lane);
@@ -881,8 +884,8 @@ void launch_vec(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT
   const int threads = 256;
   const int64_t need = (op.n * G + threads - 1) / threads;
   const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(ex.sms) * 8)));
-  k_spmm_vec<VT, XT, LD, G><<<grid, threads, 0, ex.stream>>>(op.n, op.indptr, op.indices, vals, op.diag, x, y,
-                                                              ep, stop);
+  launch_after(ex.stream, k_spmm_vec<VT, XT, LD, G>, grid, threads, 0, op.n, op.indptr, op.indices, vals, op.diag, x,
+               y, ep, stop);
   SI_LAUNCH_CHECK();
 }
 
@@ -1099,8 +1102,10 @@ __global__ void k_sell_fill(int64_t n_slices, const uint64_t* __restrict__ slice
   }
 }
 
-// x row gather for the sliced kernel: L1-cached (.nc; measured faster on
-// every operator tried) or L2-only (.cg).
+// x row gather for the sliced kernel: L1-cached (measured faster on every
+// operator tried) or L2-only (.cg).  Not the read-only path: the kernel may be
+// resident while its predecessor still writes x (kernel_begin), and a
+// read-only load may be moved up across that wait.
 template <class XT, int LD, bool L1>
 struct SellRowLoad;
 template <int LD, bool L1>
@@ -1110,7 +1115,7 @@ struct SellRowLoad<double, LD, L1> {
     for (int q = 0; q < LD / 4; ++q) {
       double a, b, c, d;
       if constexpr (L1)
-        asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p + 4 * q));
+        asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p + 4 * q));
       else
         asm volatile("ld.global.cg.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p + 4 * q));
       v[4 * q + 0] = a;
@@ -1126,7 +1131,11 @@ struct SellRowLoad<float, LD, L1> {
 #pragma unroll
     for (int q = 0; q < LD / 4; ++q) {
       const float4* a = reinterpret_cast<const float4*>(p + 4 * q);
-      const float4 t = L1 ? __ldg(a) : __ldcg(a);
+      float4 t;
+      if constexpr (L1)
+        asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "l"(a));
+      else
+        t = __ldcg(a);
       v[4 * q + 0] = t.x;
       v[4 * q + 1] = t.y;
       v[4 * q + 2] = t.z;
@@ -1166,9 +1175,8 @@ __device__ __forceinline__ void l2_prefetch_bulk(const void* p, uint32_t bytes) 
 template <class VT, class XT, int LD, int U, int NT, bool L1, bool PF, bool PIPE>
 __global__ void __launch_bounds__(NT, 1) k_spmm_sell(SellArgs a, const VT* __restrict__ sval,
                                                      const VT* __restrict__ vals, double diag,
-                                                     const XT* __restrict__ x, XT* __restrict__ y, Epilogue<XT> ep,
-                                                     const int* __restrict__ stop) {
-  if (stop != nullptr && *stop != 0) return;
+                                                     const XT* x, XT* y, Epilogue<XT> ep,
+                                                     const int* stop) {
   __shared__ long long next_long, next_slice;
   const int lane = threadIdx.x & 31;
   const uint64_t total = a.slice_ptr[a.n_slices];
@@ -1177,6 +1185,9 @@ __global__ void __launch_bounds__(NT, 1) k_spmm_sell(SellArgs a, const VT* __res
       blockIdx.x + 1 == gridDim.x ? a.n_slices : sell_bound(a.slice_ptr, a.n_slices, total * (blockIdx.x + 1) / gridDim.x);
   const int64_t l_lo = a.n_long * blockIdx.x / gridDim.x;
   const int64_t l_hi = a.n_long * (blockIdx.x + 1) / gridDim.x;
+  kernel_begin();  // the searches above read the operator's structure alone
+  if (stop != nullptr && *stop != 0) return;
+  x = after_begin(x);
   if (threadIdx.x == 0) {
     next_long = l_lo;
     next_slice = s_lo;
@@ -1401,7 +1412,8 @@ bool launch_sell(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, X
   const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(L->n_slices, int64_t(ex.sms) * resident[dev])));
   const SellArgs args{L->n_slices, L->n_long, L->slice_ptr.get(), L->perm.get(), L->plen.get(),
                       L->idx.get(), L->long_rows.get(), op.indptr, op.indices};
-  k_spmm_sell<VT, XT, LD, U, NT, L1, PF, PIPE><<<grid, NT, 0, ex.stream>>>(args, sval, vals, op.diag, x, y, ep, stop);
+  launch_after(ex.stream, k_spmm_sell<VT, XT, LD, U, NT, L1, PF, PIPE>, grid, NT, 0, args, sval, vals, op.diag, x, y,
+               ep, stop);
   SI_LAUNCH_CHECK();
   return true;
 }
