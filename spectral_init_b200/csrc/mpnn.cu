@@ -147,21 +147,37 @@ __global__ void __launch_bounds__(kT) k_mp_backward(int64_t n, const uint64_t* _
 }
 
 // ---- transpose [n x c] (pitch pin) -> [c x npad] (pitch npad), zero padded ----------
-__global__ void k_transpose_bf16(int64_t n, int c, const __nv_bfloat16* __restrict__ in, int64_t pin,
-                                 __nv_bfloat16* __restrict__ out, int64_t npad) {
-  __shared__ __nv_bfloat16 tile[32][34];
-  const int64_t r0 = static_cast<int64_t>(blockIdx.x) * 32;
-  const int c0 = blockIdx.y * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int64_t r = r0 + k;
-    const int cc = c0 + threadIdx.x;
-    tile[k][threadIdx.x] = (r < n && cc < c) ? in[r * pin + cc] : __float2bfloat16_rn(0.0f);
+// 64 x 64 tiles, 16-byte loads and stores (pitches are multiples of eight, bases
+// 16-byte aligned, as the GEMM's tensor maps ask; c is a multiple of eight).
+// 32 x 32 tiles by single elements took 13.6 us at n = 60k; this 5.7 us.
+constexpr int kTrTile = 64;
+constexpr int kTrThreads = 256;
+
+__global__ void __launch_bounds__(kTrThreads) k_transpose_bf16(int64_t n, int c, const __nv_bfloat16* __restrict__ in,
+                                                               int64_t pin, __nv_bfloat16* __restrict__ out,
+                                                               int64_t npad) {
+  __shared__ __align__(16) uint16_t tile[kTrTile][kTrTile + 2];  // [row][column]
+  const int64_t r0 = static_cast<int64_t>(blockIdx.x) * kTrTile;
+  const int c0 = blockIdx.y * kTrTile;
+  for (int t = threadIdx.x; t < kTrTile * kTrTile / 8; t += kTrThreads) {
+    const int r = t / (kTrTile / 8), q = t % (kTrTile / 8) * 8;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (r0 + r < n && c0 + q < c) v = *reinterpret_cast<const uint4*>(in + (r0 + r) * pin + c0 + q);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(&tile[r][q]);
+    dst[0] = v.x;
+    dst[1] = v.y;
+    dst[2] = v.z;
+    dst[3] = v.w;
   }
   __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int cc = c0 + k;
-    const int64_t r = r0 + threadIdx.x;
-    if (cc < c && r < npad) out[static_cast<int64_t>(cc) * npad + r] = tile[threadIdx.x][k];
+  for (int t = threadIdx.x; t < kTrTile * kTrTile / 8; t += kTrThreads) {
+    const int cc = t / (kTrTile / 8), q = t % (kTrTile / 8) * 8;
+    if (c0 + cc >= c || r0 + q >= npad) continue;
+    uint32_t w[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      w[u] = static_cast<uint32_t>(tile[q + 2 * u][cc]) | static_cast<uint32_t>(tile[q + 2 * u + 1][cc]) << 16;
+    *reinterpret_cast<uint4*>(out + static_cast<int64_t>(c0 + cc) * npad + r0 + q) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -579,10 +595,10 @@ double mpnn_loss_backward(const Exec& ex, MpnnModel& model, const OpDev& op, Mpn
       gb(kMpnnHidden, ex.stream);
   DevBuf<__nv_bfloat16> dz(static_cast<size_t>(n) * kMpnnHidden, ex.stream),
       dzt(static_cast<size_t>(kMpnnHidden) * npad, ex.stream);
-  const dim3 tblk(32, 8);
   auto transpose = [&](const __nv_bfloat16* in, int c, int64_t pin, __nv_bfloat16* out) {
-    const dim3 grid(static_cast<unsigned>((npad + 31) / 32), static_cast<unsigned>((c + 31) / 32));
-    k_transpose_bf16<<<grid, tblk, 0, ex.stream>>>(n, c, in, pin, out, npad);
+    const dim3 grid(static_cast<unsigned>((npad + kTrTile - 1) / kTrTile),
+                    static_cast<unsigned>((c + kTrTile - 1) / kTrTile));
+    k_transpose_bf16<<<grid, kTrThreads, 0, ex.stream>>>(n, c, in, pin, out, npad);
     SI_LAUNCH_CHECK();
   };
   // weight gradients reduce over all n rows: split K so every SM gets a slice of at least 1024 rows
