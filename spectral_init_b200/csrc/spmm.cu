@@ -160,12 +160,11 @@ struct SharedStream {  // entries [base, base + count) staged in shared memory
 // One row of y = epilogue(A x) by a group of G lanes.  U entries per lane per
 // pass: all index/value reads of a pass are issued before its gathers.  The
 // own-row epilogue terms are loaded first so they overlap the gathers.
-template <class VT, class XT, int LD, int G, class Src>
+template <class VT, class XT, int LD, int G, int U = (LD >= 16 ? 4 : 8), class Src>
 __device__ __forceinline__ void spmm_row(int64_t row, uint64_t s, uint64_t e, const Src& src, double diag,
                                          const XT* __restrict__ x, XT* __restrict__ y, const Epilogue<XT>& ep,
                                          int sub, unsigned mask, bool writer) {
   constexpr int W = GroupReduce<LD, G>::W;
-  constexpr int U = (LD >= 16) ? 4 : 8;
   const int obase = GroupReduce<LD, G>::base_of(sub);
   double own[W], addz[W];
 #pragma unroll
@@ -224,7 +223,14 @@ __device__ __forceinline__ bool group_writer(int sub) {
 }
 
 // Direct kernel: rows in grid-stride order, streams read from global memory;
-// the next row's bounds are fetched while the current row is in flight.
+// the next row's bounds are fetched while the current row is in flight.  Bound
+// by latency and issue: a pass of the group covers 64 entries (U = 64 / G a
+// lane, at most 8), which most rows of a neighbour graph fit, because a slot
+// without an entry still costs its instructions; U = 8 whatever the group took
+// 23.4 us at n = 60k and 43.7 at n = 120k (f32, 4 columns, 16 lanes), this 19.6
+// and 34.9; 11.6 against 9.6 at n = 20k (32 lanes).
+constexpr int vec_unroll(int g) { return 64 / g < 8 ? 64 / g : 8; }
+
 template <class VT, class XT, int LD, int G>
 __global__ void __launch_bounds__(256) k_spmm_vec(int64_t n, const uint64_t* __restrict__ indptr,
                                                   const uint32_t* __restrict__ indices,
@@ -255,7 +261,7 @@ __global__ void __launch_bounds__(256) k_spmm_vec(int64_t n, const uint64_t* __r
       ns = __ldg(indptr + nrow);
       ne = __ldg(indptr + nrow + 1);
     }
-    spmm_row<VT, XT, LD, G>(row, s, e, src, diag, x, y, ep, sub, mask, writer);
+    spmm_row<VT, XT, LD, G, vec_unroll(G)>(row, s, e, src, diag, x, y, ep, sub, mask, writer);
     s = ns;
     e = ne;
   }
@@ -883,7 +889,11 @@ void launch_vec(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT
                 const int* stop) {
   const int threads = 256;
   const int64_t need = (op.n * G + threads - 1) / threads;
-  const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(ex.sms) * 8)));
+  // Four columns: a row a group, so the scheduler levels rows of uneven length
+  // (n = 120k, f32: 34.9 us against 38.4 with eight blocks an SM striding; f64
+  // 47.1 against 47.2, 100k rows of 16 f32 columns 108.1 against 96.6).
+  const int64_t cap = LD == 4 ? INT32_MAX : int64_t(ex.sms) * 8;
+  const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(need, cap)));
   launch_after(ex.stream, k_spmm_vec<VT, XT, LD, G>, grid, threads, 0, op.n, op.indptr, op.indices, vals, op.diag, x,
                y, ep, stop);
   SI_LAUNCH_CHECK();
