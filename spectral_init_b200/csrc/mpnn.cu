@@ -59,45 +59,134 @@ __global__ void k_features(int64_t n, const double* __restrict__ sqrt_deg, doubl
 }
 
 // ---- message passing: A[:, 64:128] = Ahat A[:, 0:64] (Ahat = -offdiag(L)) -------------
+// kLanes lanes a row, sixteen bytes of the row's 64 columns each (8 lanes of bf16
+// forward, 16 of f32 backward).  Every column is summed in f32 over the row's
+// entries in order: another order moves the bf16 roundings behind it, which the
+// loss's conditioning turns into 3e-3 of a gradient.  Bound by the gathers'
+// latency: kMpUnroll entries of a row are in flight, the next ones' indices and
+// weights with them.  A row of more than kMpLong entries (a hub of a neighbour
+// graph; 675 where the mean is 24) is gathered by the whole block through shared
+// memory, or its lanes would outlast the launch.  A warp a row, one entry at a
+// time (4 or 8 bytes a lane, four in flight) took 54.4 us forward and 68.4 us
+// backward a layer at n = 60k, k = 15; this 49 and 53 (long rows from 48 or 256
+// entries on: 54.0 and 61.0, 52.8 and 51.7; eight entries in flight 48.7 and 60.0).
+constexpr int kMpUnroll = 4;
+constexpr int kMpLong = 128;
+constexpr int kMpStageBytes = 16384;
+
+__device__ __forceinline__ float mp_float(__nv_bfloat16 v) { return __bfloat162float(v); }
+__device__ __forceinline__ float mp_float(float v) { return v; }
+
+// acc -= w f, f the sixteen bytes as eight bf16 or four f32
+__device__ __forceinline__ void mp_subtract(float w, const uint4& g, float (&acc)[8]) {
+  const uint32_t b[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b[v]));
+    acc[2 * v] -= w * f.x;
+    acc[2 * v + 1] -= w * f.y;
+  }
+}
+
+__device__ __forceinline__ void mp_subtract(float w, const uint4& g, float (&acc)[4]) {
+  acc[0] -= w * __uint_as_float(g.x);
+  acc[1] -= w * __uint_as_float(g.y);
+  acc[2] -= w * __uint_as_float(g.z);
+  acc[3] -= w * __uint_as_float(g.w);
+}
+
+// finish(row, first column, start - sum_e w_e X[j_e]) for every row; X the 64 columns of T at
+// x + kMpnnCat j, start = begin(row, first column).
+template <class T, int V, class Begin, class Finish>
+__device__ __forceinline__ void mp_rows(int64_t n, const uint64_t* __restrict__ indptr,
+                                        const uint32_t* __restrict__ indices, const float* __restrict__ vals,
+                                        const T* x, const Begin& begin, const Finish& finish) {
+  constexpr int kLanes = kMpnnHidden / V, kRows = kT / kLanes;
+  constexpr int kStage = kMpStageBytes / (kMpnnHidden * static_cast<int>(sizeof(T)));
+  static_assert(V * sizeof(T) == 16 && kT >= kMpnnHidden, "sixteen bytes a lane, a thread a column");
+  __shared__ uint4 stage[kMpStageBytes / 16];
+  __shared__ float weight[kStage];
+  const int q = threadIdx.x % kLanes * V;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * kRows, row = row0 + threadIdx.x / kLanes;
+  const uint64_t e0 = row < n ? indptr[row] : 0, e1 = row < n ? indptr[row + 1] : 0;
+  const bool longer = e1 - e0 > kMpLong;
+  const bool any = __syncthreads_or(longer);
+  if (row < n && !longer) {
+    float acc[V];
+    begin(row, q, acc);
+    uint32_t j[kMpUnroll];
+    float w[kMpUnroll];
+    const uint32_t* idx = indices + e0;
+    const float* val = vals + e0;
+    const int len = static_cast<int>(e1 - e0);
+    auto entries = [&](int e) {
+#pragma unroll
+      for (int u = 0; u < kMpUnroll; ++u) {
+        j[u] = e + u < len ? __ldg(idx + e + u) : 0u;
+        w[u] = e + u < len ? __ldg(val + e + u) : 0.0f;
+      }
+    };
+    entries(0);
+    for (int e = 0; e < len; e += kMpUnroll) {
+      uint4 g[kMpUnroll];
+      float wg[kMpUnroll];
+#pragma unroll
+      for (int u = 0; u < kMpUnroll; ++u) {
+        g[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (e + u < len) g[u] = *reinterpret_cast<const uint4*>(x + static_cast<int64_t>(j[u]) * kMpnnCat + q);
+        wg[u] = w[u];
+      }
+      entries(e + kMpUnroll);
+#pragma unroll
+      for (int u = 0; u < kMpUnroll; ++u) mp_subtract(wg[u], g[u], acc);
+    }
+    finish(row, q, acc);
+  }
+  if (!any) return;
+  for (int64_t r = row0; r < min(row0 + kRows, n); ++r) {
+    const uint64_t r0 = indptr[r], r1 = indptr[r + 1];
+    if (r1 - r0 <= kMpLong) continue;
+    float acc[1] = {0.0f};
+    if (threadIdx.x < kMpnnHidden) begin(r, static_cast<int>(threadIdx.x), acc);
+    for (uint64_t e = r0; e < r1; e += kStage) {
+      const int cnt = static_cast<int>(min(r1 - e, static_cast<uint64_t>(kStage)));
+#pragma unroll 4
+      for (int t = threadIdx.x; t < cnt * kLanes; t += kT) {
+        const uint32_t j = __ldg(indices + e + t / kLanes);
+        stage[t] = *reinterpret_cast<const uint4*>(x + static_cast<int64_t>(j) * kMpnnCat + q);
+      }
+      if (threadIdx.x < cnt) weight[threadIdx.x] = __ldg(vals + e + threadIdx.x);
+      __syncthreads();
+      if (threadIdx.x < kMpnnHidden) {
+        const T* column = reinterpret_cast<const T*>(stage) + threadIdx.x;
+#pragma unroll 8
+        for (int u = 0; u < cnt; ++u) acc[0] -= weight[u] * mp_float(column[u * kMpnnHidden]);
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x < kMpnnHidden) finish(r, static_cast<int>(threadIdx.x), acc);
+  }
+}
+
 __global__ void __launch_bounds__(kT) k_mp_forward(int64_t n, const uint64_t* __restrict__ indptr,
                                                    const uint32_t* __restrict__ indices,
                                                    const float* __restrict__ vals, __nv_bfloat16* __restrict__ a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (kT / 32);
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(kT / 32) + (threadIdx.x >> 5); i < n; i += warps) {
-    const uint64_t e0 = indptr[i], e1 = indptr[i + 1];
-    float2 acc = make_float2(0.f, 0.f);
-    uint64_t e = e0;
-    for (; e + 4 <= e1; e += 4) {
-      uint32_t j[4];
-      float w[4];
-      __nv_bfloat162 h[4];
+  mp_rows<__nv_bfloat16, 8>(
+      n, indptr, indices, vals, a,
+      [](int64_t, int, auto& acc) {
+        for (float& v : acc) v = 0.0f;
+      },
+      [&](int64_t i, int c, const auto& acc) {
+        __nv_bfloat16* out = a + i * kMpnnCat + kMpnnHidden + c;
+        if constexpr (sizeof(acc) == sizeof(float)) {
+          *out = __float2bfloat16_rn(acc[0]);
+        } else {
+          __align__(16) __nv_bfloat162 o[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        j[u] = __ldg(indices + e + u);
-        w[u] = __ldg(vals + e + u);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        h[u] = *reinterpret_cast<const __nv_bfloat162*>(a + static_cast<int64_t>(j[u]) * kMpnnCat + 2 * lane);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float2 f = __bfloat1622float2(h[u]);
-        acc.x -= w[u] * f.x;
-        acc.y -= w[u] * f.y;
-      }
-    }
-    for (; e < e1; ++e) {
-      const uint32_t j = __ldg(indices + e);
-      const float w = __ldg(vals + e);
-      const float2 f = __bfloat1622float2(
-          *reinterpret_cast<const __nv_bfloat162*>(a + static_cast<int64_t>(j) * kMpnnCat + 2 * lane));
-      acc.x -= w * f.x;
-      acc.y -= w * f.y;
-    }
-    *reinterpret_cast<__nv_bfloat162*>(a + i * kMpnnCat + kMpnnHidden + 2 * lane) =
-        __floats2bfloat162_rn(acc.x, acc.y);
-  }
+          for (int v = 0; v < 4; ++v) o[v] = __floats2bfloat162_rn(acc[2 * v], acc[2 * v + 1]);
+          *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(o);
+        }
+      });
 }
 
 // ---- backward through [H | Ahat H] and the ReLU of H:
@@ -107,43 +196,34 @@ __global__ void __launch_bounds__(kT) k_mp_backward(int64_t n, const uint64_t* _
                                                     const float* __restrict__ vals, const float* __restrict__ da,
                                                     const __nv_bfloat16* __restrict__ h,
                                                     __nv_bfloat16* __restrict__ dz) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (kT / 32);
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(kT / 32) + (threadIdx.x >> 5); i < n; i += warps) {
-    const uint64_t e0 = indptr[i], e1 = indptr[i + 1];
-    float2 acc = *reinterpret_cast<const float2*>(da + i * kMpnnCat + 2 * lane);
-    uint64_t e = e0;
-    for (; e + 4 <= e1; e += 4) {
-      uint32_t j[4];
-      float w[4];
-      float2 g[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        j[u] = __ldg(indices + e + u);
-        w[u] = __ldg(vals + e + u);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        g[u] = *reinterpret_cast<const float2*>(da + static_cast<int64_t>(j[u]) * kMpnnCat + kMpnnHidden + 2 * lane);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        acc.x -= w[u] * g[u].x;
-        acc.y -= w[u] * g[u].y;
-      }
-    }
-    for (; e < e1; ++e) {
-      const uint32_t j = __ldg(indices + e);
-      const float w = __ldg(vals + e);
-      const float2 g =
-          *reinterpret_cast<const float2*>(da + static_cast<int64_t>(j) * kMpnnCat + kMpnnHidden + 2 * lane);
-      acc.x -= w * g.x;
-      acc.y -= w * g.y;
-    }
-    const float2 hv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(h + i * kMpnnCat + 2 * lane));
-    const float gx = hv.x > 0.0f ? acc.x : 0.0f;
-    const float gy = hv.y > 0.0f ? acc.y : 0.0f;
-    *reinterpret_cast<__nv_bfloat162*>(dz + i * kMpnnHidden + 2 * lane) = __floats2bfloat162_rn(gx, gy);
-  }
+  mp_rows<float, 4>(
+      n, indptr, indices, vals, da + kMpnnHidden,
+      [&](int64_t i, int c, auto& acc) {
+        if constexpr (sizeof(acc) == sizeof(float)) {
+          acc[0] = da[i * kMpnnCat + c];
+        } else {
+          const float4 own = *reinterpret_cast<const float4*>(da + i * kMpnnCat + c);
+          acc[0] = own.x;
+          acc[1] = own.y;
+          acc[2] = own.z;
+          acc[3] = own.w;
+        }
+      },
+      [&](int64_t i, int c, const auto& acc) {
+        const __nv_bfloat16* hr = h + i * kMpnnCat + c;
+        __nv_bfloat16* out = dz + i * kMpnnHidden + c;
+        if constexpr (sizeof(acc) == sizeof(float)) {
+          *out = __float2bfloat16_rn(__bfloat162float(*hr) > 0.0f ? acc[0] : 0.0f);
+        } else {
+          const uint2 hb = *reinterpret_cast<const uint2*>(hr);
+          const float2 h0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hb.x));
+          const float2 h1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hb.y));
+          __align__(8) __nv_bfloat162 o[2];
+          o[0] = __floats2bfloat162_rn(h0.x > 0.0f ? acc[0] : 0.0f, h0.y > 0.0f ? acc[1] : 0.0f);
+          o[1] = __floats2bfloat162_rn(h1.x > 0.0f ? acc[2] : 0.0f, h1.y > 0.0f ? acc[3] : 0.0f);
+          *reinterpret_cast<uint2*>(out) = *reinterpret_cast<const uint2*>(o);
+        }
+      });
 }
 
 // ---- transpose [n x c] (pitch pin) -> [c x npad] (pitch npad), zero padded ----------
@@ -542,7 +622,7 @@ void mpnn_features(const Exec& ex, const OpDev& op, const double* sqrt_deg, uint
 
 void mpnn_forward(const Exec& ex, const MpnnModel& model, const OpDev& op, MpnnActs& acts, GemmWorkspace& ws) {
   const int64_t n = op.n;
-  const int gmp = grid_for_rows(ex, n * 32, 16);
+  const unsigned gmp = static_cast<unsigned>((n + kT / 8 - 1) / (kT / 8));  // eight lanes a row
   for (int l = 0; l <= kMpnnLayers; ++l) {
     k_mp_forward<<<gmp, kT, 0, ex.stream>>>(n, op.indptr, op.indices, op.v32, acts.a[l].get());
     SI_LAUNCH_CHECK();
@@ -624,7 +704,7 @@ double mpnn_loss_backward(const Exec& ex, MpnnModel& model, const OpDev& op, Mpn
     gemm_bf16_nt(ex, n, kMpnnCat, kMpnnOut, dy.get(), kMpnnOut,
                  model.w.get() + static_cast<int64_t>(kMpnnLayers) * kMpnnHidden * kMpnnCat, kMpnnOut, ed, 1, ws);
   }
-  const int gmp = grid_for_rows(ex, n * 32, 16);
+  const unsigned gmp = static_cast<unsigned>((n + kT / 16 - 1) / (kT / 16));  // sixteen lanes a row
   for (int l = kMpnnLayers - 1; l >= 0; --l) {
     // dZ_l from dA_{l+1} through the message passing and the ReLU of H_{l+1}
     k_mp_backward<<<gmp, kT, 0, ex.stream>>>(n, op.indptr, op.indices, op.v32, da.get(), acts.a[l + 1].get(),

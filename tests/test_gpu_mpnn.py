@@ -65,6 +65,35 @@ def test_gradient_matches_cpu_oracle(gpu_ctx, model_seed):
     model.close()
 
 
+@pytest.mark.parametrize("hub", [3, 128, 129, 320, 385])
+def test_gradient_with_rows_at_the_block_split(gpu_ctx, hub, monkeypatch):
+    """Rows of up to 128 entries are summed by their own lanes, longer ones by
+    the whole block through shared memory (64 or 128 entries a stage): rows on
+    both sides of each edge, in a graph of odd size, to the bounds above."""
+    import torch
+    from spectral_init_b200.warm_start import WarmStartModel
+    n = 389
+    rng = np.random.default_rng(hub)
+    rows, cols = list(range(n)), [(i + 1) % n for i in range(n)]
+    for row in (0, 200, n - 1):
+        others = rng.permutation(np.setdiff1d(np.arange(n), [(row - 1) % n, row, (row + 1) % n]))[:hub - 2]
+        rows += [row] * len(others)
+        cols += list(others)
+    g = sp.csr_matrix((rng.uniform(0.2, 1.0, len(rows)), (rows, cols)), shape=(n, n))
+    g = g.maximum(g.T).tocsr().astype(np.float32)
+    monkeypatch.setitem(_setup.__globals__, "load_graph", lambda name: g)
+    lap, target, v, ahat = _setup(gpu_ctx)
+    feats = rng.standard_normal((lap.n, M.FEATURES)).astype(np.float32)
+    model = WarmStartModel(3, ctx=gpu_ctx)
+    loss_gpu, grad_gpu = model.gradient(lap, target, features=torch.from_numpy(feats).to("cuda:0"))
+    loss_cpu, grad_cpu = M.loss_and_grad(model.get_params(), ahat, feats, v, 3, rounding=True)
+    assert abs(loss_gpu - loss_cpu) <= 1e-3 * abs(loss_cpu), (loss_gpu, loss_cpu)
+    for i, (gg, c) in enumerate(zip(_blocks(grad_gpu.astype(np.float64)), _blocks(grad_cpu))):
+        nrm = np.linalg.norm(c)
+        assert np.linalg.norm(gg - c) <= 2e-2 * max(nrm, 1e-12), (i, np.linalg.norm(gg - c), nrm)
+    model.close()
+
+
 def test_prediction_matches_oracle_forward(gpu_ctx):
     import torch
     from spectral_init_b200.warm_start import WarmStartModel
