@@ -206,7 +206,7 @@ si_status si_spmm_f32(si_ctx* ctx, const si_operator* op, const float* x, float*
 /* A device operator prepared for repeated products (the crate's CsrOperator,
  * src/operator.rs:174-228, holds its matrix across LinearOperator::apply
  * calls): the row partitions of the tiled / gather / panel kernels are built
- * once; the sliced copy of the operator (the kernel of operators of 2^22 or
+ * once; the sliced copy of the operator (the kernel of operators of 2^21 or
  * more entries, about the size of the index and value arrays again) with it, the
  * panel kernel's x windows on first use, outside stream capture.  The
  * operator's arrays must stay allocated and unchanged while the plan lives,

@@ -1485,6 +1485,7 @@ struct TuneKey {
 std::mutex g_tune_mu;
 std::map<TuneKey, int> g_tune;
 constexpr int64_t kTuneMinNnz = int64_t(1) << 22;  // operators the autotuner times
+constexpr int64_t kSlicedMinNnz = int64_t(1) << 21;  // operators whose rule asks for the sliced kernels
 
 // Tuning file (SPECTRAL_INIT_SPMM_TUNE_FILE): choices keyed by the operator's
 // shape rather than its addresses, one line "n nnz ld vbytes xbytes tiled
@@ -1560,18 +1561,20 @@ int forced_choice(const OpDev& op, bool tiled) {
 // pass more than it gains (13 candidates: 36 ms of a 77 ms first solve at n =
 // 1M, 4.9 ms before a product of 90 us at n = 300k); operators prepared with a
 // tuning file still do.  The sliced kernels, where the operator allows its
-// copy, from the size at which they beat the best CSR vector kernel (us, sliced
-// against vector; f64, 4 columns: 27 / 24 with 1.4 M entries, 54 / 75 with 4.9
-// M, 160 / 219 with 24 M; f32 alike), with the next slice prefetched while x
-// is small (57 / 54 without / with at n = 100k, 160 / 168 at n = 1M).  Wider
-// rows gain from them only once the block outgrows the L2's reach (8 columns,
-// f64: 84 / 84 with 4.9 M, 312 / 354 at n = 1M; 16 columns, f32: 140 / 113 and
-// 480 / 541), and 16 f64 columns gain nothing clear (780 / 710 in cluster order,
-// 805 / 827 shuffled; four passes of four columns: 1051 and 1182).
+// copy, from the size at which they beat the CSR vector kernel (us, sliced
+// against vector, 4 columns; f64: 22 / 26 with 1.4 M entries, 33 / 49 with 2.9 M,
+// 54 / 75 with 4.9 M, 160 / 219 with 24 M; f32: 21 / 20, 29 / 35 with 1.4 and 2.9
+// M) and a solve earns the copy back (n = 100k to 150k, 2.1 to 3.9 M entries: 2 to
+// 30 % less a solve), with the next slice prefetched while x is small (57 / 54
+// without / with at n = 100k, 160 / 168 at n = 1M).  Wider rows gain from them
+// only once the block outgrows the L2's reach (8 columns, f64: 84 / 84 with 4.9
+// M, 312 / 354 at n = 1M; 16 columns, f32: 140 / 97 and 480 / 541), and 16 f64
+// columns gain nothing clear (780 / 710 in cluster order, 805 / 827 shuffled;
+// four passes of four columns: 1051 and 1182).
 template <class VT, class XT, int LD>
 int ruled_choice(const OpDev& op) {
   const bool large = op.n >= int64_t(1) << 19;
-  if (op.panels->sell_ok && op.nnz >= kTuneMinNnz) {
+  if (op.panels->sell_ok && op.nnz >= kSlicedMinNnz) {
     if (LD == 4) return large ? 402 : 403;
     if (large) {
       if (std::is_same<XT, float>::value) return 403;
@@ -1725,7 +1728,7 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
 }  // namespace
 
 void build_sliced_copy(const Exec& ex, const OpDev& op) {
-  if (op.nnz >= kTuneMinNnz) sell_layout(ex, op);
+  if (op.nnz >= kSlicedMinNnz) sell_layout(ex, op);
 }
 
 void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok) {
