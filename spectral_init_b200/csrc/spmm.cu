@@ -1529,7 +1529,7 @@ void tune_file_append(const TuneKey& k, int choice) {  // caller holds g_tune_mu
 // Kernel override for tuning and tests: SPECTRAL_INIT_SPMM_KERNEL = vec4 | vec8 |
 // vec16 | vec32 | tiled4 | tiled8 | gather4 | gather8 | panel | sell | sell_pf | sell_pipe |
 // sell_pf_pipe (unset or "auto": the
-// autotuner).  A choice the operator or the types cannot use is ignored.
+// rule).  A choice the operator or the types cannot use is ignored.
 template <class VT, class XT, int LD>
 int forced_choice(const OpDev& op, bool tiled) {
   // SPECTRAL_INIT_SPMM_KERNEL_F32 / _F64 override it for one value type
