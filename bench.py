@@ -551,7 +551,7 @@ def _run_ours_body(a, rank, world, local, dev, barrier, max_over_ranks):
         "spmm": {"ms_f64": ms64, "ms_f32": ms32, "gbs_f64": gbs64, "gbs_f32": gbs32,
                  "algorithmic_bytes_f64": bytes64, "algorithmic_bytes_f32": bytes32,
                  "bytes_formula": "nnz*(4 idx + s_val) + (n+1)*8 indptr + 2*n*4*s_x (x read, y written; 4 columns)"},
-        "roofline": {"bound": "hbm", "kernel": "f32 SpMM, 4 columns (the autotuned kernel; ncu summary in profiles/)",
+        "roofline": {"bound": "hbm", "kernel": "f32 SpMM, 4 columns (the sliced kernel; ncu summary in profiles/)",
                      "achieved": gbs32, "peak": hbm, "unit": "GB/s", "frac": gbs32 / hbm,
                      "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peak_src == "measured"
                      else "fallback 6.65 TB/s", "traffic": traffic},
