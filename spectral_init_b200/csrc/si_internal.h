@@ -166,7 +166,7 @@ template <class XT>
 void spmm_dev(const Exec& ex, const OpDev& op, const XT* x, XT* y, int ld, int k, const Epilogue<XT>& ep,
               const int* stop = nullptr, bool use_f32_values = false);
 // Rows per group chosen for the operator's degree profile.
-int spmm_group_lanes(const OpDev& op, int ld);
+int spmm_group_lanes(const OpDev& op, int ld, bool f64);
 
 // ---- block_ops.cu -----------------------------------------------------------
 constexpr int MAXM = 16;   // widest LOBPCG block

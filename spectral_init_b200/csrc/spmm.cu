@@ -1434,7 +1434,7 @@ void launch_lanes(int g, const Exec& ex, const OpDev& op, const VT* vals, const 
                   const int* stop) {
   if (g == 300) {
     if (launch_panel<VT, XT, LD>(ex, op, vals, x, y, ep, stop)) return;
-    g = spmm_group_lanes(op, LD);  // no windows (inside a capture before first use): direct kernel
+    g = spmm_group_lanes(op, LD, sizeof(XT) == 8);  // no windows (inside a capture before first use): direct kernel
   }
   if (g >= 400 && g <= 403) {
     bool ok = false;
@@ -1445,7 +1445,7 @@ void launch_lanes(int g, const Exec& ex, const OpDev& op, const VT* vals, const 
       default: ok = launch_sell<VT, XT, LD, true, true, true>(ex, op, vals, x, y, ep, stop); break;
     }
     if (ok) return;
-    g = spmm_group_lanes(op, LD);  // no sliced copy: direct kernel
+    g = spmm_group_lanes(op, LD, sizeof(XT) == 8);  // no sliced copy: direct kernel
   }
   switch (g) {
     case 4: launch_vec<VT, XT, LD, 4>(ex, op, vals, x, y, ep, stop); break;
@@ -1581,7 +1581,7 @@ int ruled_choice(const OpDev& op) {
       if (LD == 8) return 401;
     }
   }
-  return spmm_group_lanes(op, LD);
+  return spmm_group_lanes(op, LD, sizeof(XT) == 8);
 }
 
 // Blocks whose row stride or alignment the vector gathers cannot take: packed
@@ -1646,7 +1646,7 @@ void dispatch_g(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT
     // below ~4 M stored entries timing the candidates (and building the
     // sliced copy for them) costs more than a better kernel saves
     if (cs != cudaStreamCaptureStatusNone || op.nnz < kTuneMinNnz) {
-      g = spmm_group_lanes(op, LD);
+      g = spmm_group_lanes(op, LD, sizeof(XT) == 8);
     } else {
       timed = true;
       cudaEvent_t e0, e1;
@@ -1717,7 +1717,7 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
       return;
     }
   }
-  switch (spmm_group_lanes(op, 4)) {
+  switch (spmm_group_lanes(op, 4, sizeof(XT) == 8)) {
     case 4: return launch_generic<VT, XT, 4>(ex, op, vals, x, y, ld, k, ep, stop);
     case 8: return launch_generic<VT, XT, 8>(ex, op, vals, x, y, ld, k, ep, stop);
     case 16: return launch_generic<VT, XT, 16>(ex, op, vals, x, y, ld, k, ep, stop);
@@ -1763,17 +1763,25 @@ void make_row_blocks(const Exec& ex, const OpDev& op, RowBlocks& rb) {
   rb.sell_failed = false;
 }
 
-int spmm_group_lanes(const OpDev& op, int ld) {
-  // A lane covers up to 8 entries per pass: the fewest lanes that keep most
-  // rows to one pass, since more rows in flight per SM beats wider groups --
-  // as long as there are rows enough to fill the GPU.  Below half a million
-  // lanes wider groups win (f64, 4 columns, us with 4 / 8 / 16 / 32 lanes: 31 /
-  // 29 / 18 / 15 at n = 20 000, 31 / 31 / 24 / 27 at 60 000, 77 / 78 / 71 / 89
-  // at 200 000); 8 and 16 columns leave a lane enough columns to reduce only
-  // from 16 lanes on (16 columns at n = 60 000: 82 / 74 / 57 / 64).
+int spmm_group_lanes(const OpDev& op, int ld, bool f64) {
+  // Few lanes a row keep more rows in flight per SM, many end a long row
+  // sooner, which counts as long as the GPU is not full (us with 4 / 8 / 16 / 32
+  // lanes, 4 columns, k = 15; f32: 41 / 32 / 24 / 31 at n = 75 000, 84 / 70 / 60 /
+  // 83 at 200 000, 128 / 124 / 143 / 201 at 600 000; f64: 33 / 30 / 20 / 12 at
+  // 20 000, 36 / 33 / 30 / 30 at 75 000, 134 / 138 / 167 / 214 at 600 000; k = 5,
+  // f32: 16 / 13 / 15 / 22 at 75 000, 31 / 31 / 36 / 56 at 200 000; k = 30, n =
+  // 40 000: 61 / 46 / 27 / 31 in f32, 72 / 62 / 40 / 26 in f64).  8 and 16
+  // columns leave a lane enough columns to reduce only from 16 lanes on, but for
+  // 16 f64 columns of many rows (n = 100 000, k = 30: 123 / 135 with 8 / 16 lanes;
+  // 400 000, k = 15: 237 / 277).
   const double mean = op.n > 0 ? static_cast<double>(op.nnz) / static_cast<double>(op.n) : 0.0;
   int g = mean <= 28.0 ? 4 : (mean <= 56.0 ? 8 : (mean <= 112.0 ? 16 : 32));
-  if (ld >= 8) g = std::max(g, 16);
+  if (ld >= 8) {
+    g = std::max(g, ld == 16 && f64 && op.n >= int64_t(1) << 16 ? 8 : 16);
+  } else if (mean > 12.0) {
+    while (g < 16 && op.n * g < int64_t(1) << 21) g *= 2;
+    if (f64 && op.n < int64_t(1) << 16) g = 32;
+  }
   while (g < 32 && op.n * g < int64_t(1) << 19) g *= 2;
   return g;
 }
