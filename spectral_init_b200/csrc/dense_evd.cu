@@ -197,11 +197,17 @@ __global__ void k_tri_last(const double* A, int n, double* d, double* e, double*
 //   Otherwise (cooperative launch, up to one CTA an SM): pairs go through L2
 //   as 16-byte words (value, step number), stored and loaded as single 128-bit
 //   accesses, so that a word carries its own arrival flag and nothing has to be
-//   ordered against it.  Words are double-buffered by step parity: a word is
-//   rewritten two steps later, after its owner has seen step j + 1 of every
-//   CTA, each of which had read step j by then.  Every wait is bounded: a
-//   thread that waits longer than the limit sets the error word, every CTA
-//   returns, and the host redoes the matrix with the multi-launch steps.
+//   ordered against it.  Words are double-buffered by step parity, and a word
+//   is rewritten two steps later.  Its readers at step j are the CTAs with a row
+//   > j.  Each of them has a row >= j + 1 and publishes it at step j + 1, after
+//   its reads of step j; the gather of step j + 1 waits for the words of all rows
+//   >= j + 1, so nobody is at step j + 2 before.  The word of row j + 1 itself
+//   holds nothing then: it says that its owner is through step j, which no other
+//   word may (a CTA whose last row is j + 1 has none below).  With it published
+//   and the reflector stored, a CTA whose rows are all finished leaves.  Every
+//   wait is bounded: a thread that waits longer than the limit sets the error
+//   word, every CTA returns, and the host redoes the matrix with the
+//   multi-launch steps.
 constexpr int CT_THREADS = 256;
 constexpr int CT_WARPS = CT_THREADS / 32;
 constexpr int CT_CHUNK = 16;                                     // rows a pass accumulates at a time
@@ -397,14 +403,15 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
         *cooperative_groups::this_cluster().map_shared_rank(pairs + (j & 1) * n + l * G + b, peer) =
             make_double2(sum, rows[l * ns + j + 1]);
       }
-    } else if (tid < nl) {
-      const int l = l0 + tid;
+    } else if (tid < nl + (owner ? 1 : 0)) {
+      const bool done = tid == nl;  // row j, in slot l0 - 1
+      const int l = done ? l0 - 1 : l0 + tid;
       double sum = 0.0;
 #pragma unroll
       for (int w = 0; w < CT_WARPS; ++w) sum += pr[w][l];
       ulonglong2* out = p.words + (static_cast<size_t>(j & 1) * n + l * G + b) * 2;
-      st_word(out, sum, step);
-      st_word(out + 1, rows[l * ns + j + 1], step);
+      st_word(out, done ? 0.0 : sum, step);
+      st_word(out + 1, done ? 0.0 : rows[l * ns + j + 1], step);
     }
     const double tau = tau_inv != 0.0 ? 1.0 / tau_inv : 0.0;
     // Row j of A takes the reflector, normalised to a first element of one as
@@ -424,6 +431,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
       }
     };
     if (j > 0) keep_reflector();
+    if (!CLUSTER && nl == 0) return;  // j > 0 here: every CTA starts with three rows or more
     // gather
     double pc[CMAX], ac[CMAX];
     int fail = 0;
@@ -444,7 +452,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
         const int c = tid + q * CT_THREADS;
         pc[q] = 0.0;
         ac[q] = 0.0;
-        if (c > j && c < n) missing |= 1u << q;
+        if (c >= j && c < n) missing |= 1u << q;
       }
       uint64_t t0 = 0;
       unsigned fails = 0;
