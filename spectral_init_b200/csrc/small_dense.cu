@@ -141,8 +141,11 @@ __device__ double cta_sum(double v, double* red) {
 // A and V stay exactly similar / orthogonal, and an angle off by ~1e-7 only
 // leaves ~1e-7 of a_pq for the next sweep (quadratic convergence down to that
 // level, then a factor ~1e-7 per sweep).  No f64 square root or division on
-// the round's critical path.  On return A (diagonal) and V hold the result.
-__device__ void cta_jacobi_db(double* A, double* V, double* A2, double* V2, int s, int ld, double* red) {
+// the round's critical path.  The single-precision angle and the sums of
+// squares want entries of order one: A is scaled by a power of two (exact)
+// first.  On return A's diagonal and V hold the result; false, with nothing
+// done, where A is not finite.
+__device__ bool cta_jacobi_db(double* A, double* V, double* A2, double* V2, int s, int ld, double* red) {
   __shared__ double al[3 * MAXM + 2], be[3 * MAXM + 2];
   __shared__ int pq[3 * MAXM + 2];
   constexpr int kItems = 9;  // per-thread update items resolved once when 2 s^2 <= 9 * threads
@@ -158,6 +161,25 @@ __device__ void cta_jacobi_db(double* A, double* V, double* A2, double* V2, int 
     it_i[q] = u / s;
     it_j[q] = u - (u / s) * s;
   }
+  double big = 0.0;
+  int bad = 0;
+  for (int t = threadIdx.x; t < s * s; t += blockDim.x) {
+    const int i = t / s, j = t - (t / s) * s;
+    const double a = fabs(A[i * ld + j]);
+    big = fmax(big, a);
+    if (!(a <= DBL_MAX)) bad = 1;
+  }
+  big = warp_max(big);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = big;
+  if (__syncthreads_or(bad)) return false;
+  for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) big = fmax(big, red[i]);
+  const int ex = min(max(__double2hiint(big) >> 20, 1), 2045);  // exponent field
+  const double sc = __hiloint2double((2046 - ex) << 20, 0), unscale = __hiloint2double(ex << 20, 0);
+  for (int t = threadIdx.x; t < s * s; t += blockDim.x) {
+    const int i = t / s, j = t - (t / s) * s;
+    A[i * ld + j] *= sc;
+  }
+  __syncthreads();
   double* cur = A;
   double* nxt = A2;
   double* vc = V;
@@ -253,8 +275,11 @@ __device__ void cta_jacobi_db(double* A, double* V, double* A2, double* V2, int 
       A[i * ld + j] = cur[i * ld + j];
       V[i * ld + j] = vc[i * ld + j];
     }
+    __syncthreads();
   }
+  for (int i = threadIdx.x; i < s; i += blockDim.x) A[i * ld + i] *= unscale;
   __syncthreads();
+  return true;
 }
 
 // Parallel cyclic Jacobi (round-robin pairing): A <- diag, V <- eigenvectors
@@ -479,8 +504,11 @@ __device__ bool cta_rr_general(const double* gb, const double* ga, int P, const 
   __syncthreads();
   cta_identity(sm.V, s, ld);
   __syncthreads();
-  if (s <= 3 * MAXM) cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red);
-  else cta_jacobi(sm.A, sm.V, s, ld, red, rc, rs, ra, rb);
+  if (s <= 3 * MAXM) {
+    if (!cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red)) return false;
+  } else {
+    cta_jacobi(sm.A, sm.V, s, ld, red, rc, rs, ra, rb);
+  }
   if (threadIdx.x == 0) {
     sort_eigs(sm.A, s, ld, order);
     if (largest) {
@@ -720,6 +748,21 @@ __device__ bool warp_rr_general(const double* gb, const double* ga, int P, const
     for (int i = 0; i < WRR; ++i) col[i] = (i == j) ? 1.0 : 0.0;  // V = I
   }
   __syncwarp();
+  // a power of two to entries of order one, as in cta_jacobi_db
+  double big = 0.0;
+  bad = 0;
+#pragma unroll
+  for (int i = 0; i < WRR; ++i) {
+    big = isv ? big : fmax(big, fabs(col[i]));
+    if (!(fabs(col[i]) <= DBL_MAX)) bad = 1;
+  }
+  if (__any_sync(full, bad)) return false;
+  big = warp_max(big);
+  const int ex = min(max(__double2hiint(big) >> 20, 1), 2045);
+  const double sc = __hiloint2double((2046 - ex) << 20, 0);
+#pragma unroll
+  for (int i = 0; i < WRR; ++i)
+    if (!isv) col[i] *= sc;
   const int src_lane = (isv ? WRR : 0) + kJacSigmaInv[j];
   for (int sweep = 0; sweep < 40; ++sweep) {
     double off = 0.0, dia = 0.0;
@@ -739,7 +782,7 @@ __device__ bool warp_rr_general(const double* gb, const double* ga, int P, const
     warp_jacobi_sweep(col, j, isv, src_lane);
   }
   // eigenvalues (the diagonal) ranked among the live columns
-  const double lam = isv ? 0.0 : sel16(col, j);
+  const double lam = isv ? 0.0 : sel16(col, j) * __hiloint2double(ex << 20, 0);
   int rank = 0;
 #pragma unroll
   for (int i = 0; i < WRR; ++i) {
@@ -1463,7 +1506,8 @@ __device__ bool cta_rr_general_par(const double* gb, const double* ga, int P, co
       }
     }
     __syncthreads();
-    cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red);
+    // (a C that is not finite has no order: the ranks below would not cover it)
+    if (!cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red)) return false;
     // ---- selection by ranks (ascending, or descending for `largest`; ties by index) ----
     for (int i = threadIdx.x; i < s; i += nt) {
       const double di = sm.A[i * ld + i];

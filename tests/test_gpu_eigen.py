@@ -360,3 +360,42 @@ def test_lobpcg_spmm_variants_agree(gpu_ctx, monkeypatch, kernel, precision):
     assert level == 1
     assert np.all(np.abs(vals - w) < 1e-10), (vals, w)
     assert O.max_eigenpair_residual(lap, vals, vecs) < 1e-9
+
+
+@pytest.mark.parametrize("small", ["cta", "serial", "warp", "reg"])
+@pytest.mark.parametrize("scale", [1e-100, 1e-80, 1e-60, 1e-30])
+def test_lobpcg_on_a_tiny_operator(gpu_ctx, monkeypatch, scale, small):
+    """A Laplacian times a small number: the projected matrices are outside the
+    range of the single-precision rotation angles.  The relative residual that is
+    asked for bounds the eigenvalues' error quadratically (1e-18 over the gap of
+    the wanted pairs, above 1e-6 here), which leaves rounding.  At 1e-100 the
+    products of the residuals with the operator, (1e-9 scale)^2 scale, leave the
+    range of doubles: that solve may end without pairs, but not with others."""
+    import spectral_init_b200 as si
+    monkeypatch.setenv("SPECTRAL_INIT_SMALL_STEP", small)
+    lap = load_csr("blobs_connected_200", "comp_b_laplacian.npz")
+    cfg = si.SpectralInitConfig(tol=1e-9 * scale, max_iterations=400)
+    r = si.lobpcg_solve((lap * scale).tocsr(), 2, 42, False, np.ones(lap.shape[0]), cfg, ctx=gpu_ctx)
+    if r is None:
+        assert scale == 1e-100
+        return
+    (vals, vecs), _ = r
+    want = np.linalg.eigvalsh(lap.toarray())[:3]
+    assert np.max(np.abs(vals / scale - want)) < 1e-10
+    assert np.max(np.abs(vecs.T @ vecs - np.eye(3))) < 1e-10
+
+
+@pytest.mark.parametrize("small", ["cta", "serial", "warp", "reg"])
+@pytest.mark.parametrize("block", [0, 16])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_lobpcg_refuses_an_operator_that_is_not_finite(gpu_ctx, monkeypatch, value, block, small):
+    """One entry that is not finite: the projected matrix has no eigenpairs to
+    rank, the solve ends without any and the context stays usable."""
+    import spectral_init_b200 as si
+    monkeypatch.setenv("SPECTRAL_INIT_SMALL_STEP", small)
+    lap = load_csr("blobs_connected_200", "comp_b_laplacian.npz").copy()
+    lap.data[7] = value
+    cfg = si.SpectralInitConfig(block_size=block)
+    assert si.lobpcg_solve(lap, 2, 42, False, np.ones(lap.shape[0]), cfg, ctx=gpu_ctx) is None
+    good = load_csr("blobs_connected_200", "comp_b_laplacian.npz")
+    assert si.lobpcg_solve(good, 2, 42, False, np.ones(good.shape[0]), ctx=gpu_ctx) is not None
