@@ -322,10 +322,15 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_tridiag_coop(CoopTri p) {
       sigma += t.x + t.y;
     }
     // H = I - tau v v^T, v = S (alpha - beta, x_{j+2}, ..) unnormalised: its
-    // division is not needed before w.  S, a power of two, keeps the products
-    // of a nearly zero column out of the underflow range.
-    const double S = sigma < 0x1p-700 ? 0x1p400 : 1.0;
+    // division is not needed before w.  S, a power of two from the exponents of
+    // alpha and sigma (beta's square root is not waited for), puts the column's
+    // norm into [1, 3) and v's first element into [1, 5), so that tau^2 is in
+    // range whatever the column's size (a sigma below the normal numbers leaves
+    // them above 2^-26).
     const double alpha = s_alpha;
+    const int ea = (__double2hiint(alpha) >> 20 & 0x7ff) - 1023;
+    const int eg = ((__double2hiint(sigma) >> 20 & 0x7ff) - 1023) >> 1;
+    const double S = __hiloint2double((1023 - min(max(ea, eg), 1022)) << 20, 0);
     double beta = alpha, v1 = 0.0, tau_inv = 0.0;
     if (sigma > 0.0) {
       const double nrm = sqrt(fma(alpha, alpha, sigma));

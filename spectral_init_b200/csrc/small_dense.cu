@@ -1111,10 +1111,14 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
     for (int i = lane; i < s; i += 32)
       b = fmax(b, fabs(d[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < s ? fabs(e[i]) : 0.0));
     b = warp_max(b);
-    // exponent field of b, kept where 2^-ex is a normal number (a bound outside
-    // that range, or none, leaves T unscaled: the tests below then decide)
+    // Bounds of 2^+-240 and beyond are left to the caller's Jacobi iteration: a
+    // column of norm 2^256 would take tau^2 out of range, and what the reflectors
+    // dropped (norms below 2^-465) is no longer nothing beside a bound of 2^-400.
+    // A column whose tau^2 overflows (a norm below 2^-256 beside a bound in
+    // range) leaves T without finite entries, which the tests below refuse.
     const int be = (__double2hiint(b) >> 20) & 0x7ff;
-    const int ex = be > 32 && be < 2014 ? be - 1022 : 0;
+    const bool fit = be > 1023 - 240 && be < 1023 + 240;
+    const int ex = fit ? be - 1022 : 0;
     const double sc = __hiloint2double((1023 - ex) << 20, 0);
     __syncwarp();
     for (int i = lane; i < ((s + 3) & ~3); i += 32) {
@@ -1126,9 +1130,10 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
       d[i] *= sc;
       if (i + 1 < s) e[i] *= sc;
     }
-    if (lane == 0) sscale = __hiloint2double((1023 + ex) << 20, 0);
+    if (lane == 0) sscale = fit ? __hiloint2double((1023 + ex) << 20, 0) : 0.0;
   }
   __syncthreads();
+  if (sscale == 0.0) return false;
   // ---- eigenvalues and vectors, one warp each ----
   double2* Lp = reinterpret_cast<double2*>(work) + warp * 2 * kTriMax;  // per warp: two rows
   for (int q = warp; q < nsel; q += nw) {

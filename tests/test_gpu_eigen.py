@@ -399,3 +399,35 @@ def test_lobpcg_refuses_an_operator_that_is_not_finite(gpu_ctx, monkeypatch, val
     assert si.lobpcg_solve(lap, 2, 42, False, np.ones(lap.shape[0]), cfg, ctx=gpu_ctx) is None
     good = load_csr("blobs_connected_200", "comp_b_laplacian.npz")
     assert si.lobpcg_solve(good, 2, 42, False, np.ones(good.shape[0]), ctx=gpu_ctx) is not None
+
+
+def _extreme_columns(kind, n):
+    """Symmetric matrices whose columns leave the range in which squares of
+    squares are representable."""
+    rng = np.random.default_rng(n)
+    if kind.startswith("scale"):
+        a = rng.standard_normal((n, n))
+        return (a + a.T) / 2 * float(kind[5:])
+    if kind == "far":  # one entry of 1e-120 beside a subdiagonal of order one
+        a = np.diag(2.0 + np.arange(n)) + np.diag(np.ones(n - 1), 1) + np.diag(np.ones(n - 1), -1)
+        a[0, n - 1] = a[n - 1, 0] = 1e-120
+        return a
+    x = np.sort(rng.uniform(0.0, 9.0 if kind == "kernel" else 2.0 * n, n))  # sorted points of a Gaussian kernel
+    return np.exp(-0.5 * (x[:, None] - x[None, :]) ** 2 * (8.0 if kind == "kernel" else 1.0))
+
+
+@pytest.mark.parametrize("n", [3, 12, 40, 300, 512, 513, 700])
+@pytest.mark.parametrize("kind", ["far", "kernel", "sparse kernel", "scale1e-100", "scale1e-80", "scale1e-40",
+                                  "scale1e40", "scale1e100"])
+def test_dense_evd_columns_of_any_size(gpu_ctx, kind, n):
+    """Reflectors of columns far below or above one (both kinds of launch, n <=
+    512 and above) against LAPACK, to the bound of the edge test times the norm."""
+    import spectral_init_b200 as si
+    a = _extreme_columns(kind, n)
+    norm = np.linalg.norm(a, 2)
+    k = min(4, n)
+    vals, vecs = si.dense_evd(sp.csr_matrix(a), k, ctx=gpu_ctx)
+    want = np.linalg.eigvalsh(a / norm)[:k]
+    assert np.max(np.abs(vals / norm - want)) < 1e-11
+    assert np.max(np.abs(vecs.T @ vecs - np.eye(k))) < 1e-11
+    assert np.max(np.abs(a / norm @ vecs - vecs * (vals / norm))) < 1e-11
