@@ -56,6 +56,10 @@ auto with_copy(const Exec& ex, const OpDev& op_in, SolverStats& st, F&& solve) {
   attach_ruled(ex, op, rb, true);
   const SolverStats before = st;
   try {
+    if (copy_oom_seam("solve")) {
+      build_sliced_copy(ex, op);
+      throw Error(SI_OUT_OF_MEMORY, "solve: out of memory (test seam)");
+    }
     return solve(op);
   } catch (const Error& e) {
     if (e.code != SI_OUT_OF_MEMORY || !rb.sell) throw;

@@ -1316,6 +1316,11 @@ __global__ void __launch_bounds__(NT, 1) k_spmm_sell(SellArgs a, const VT* __res
 
 }  // namespace
 
+bool copy_oom_seam(const char* where) {
+  const char* v = std::getenv("SPECTRAL_INIT_COPY_OOM");
+  return v != nullptr && std::string(v) == where;
+}
+
 uint64_t free_memory_quarter() {
   size_t free_b = 0, total_b = 0;
   SI_CUDA(cudaMemGetInfo(&free_b, &total_b));
@@ -1324,15 +1329,8 @@ uint64_t free_memory_quarter() {
 
 namespace {
 
-// The sliced-ELL copy of the operator (built on first use, outside stream
-// capture, for owners that allow it; null when not available).
-const SellLayout* sell_layout(const Exec& ex, const OpDev& op) {
-  if (op.panels == nullptr || !op.panels->sell_ok || op.panels->sell_failed) return nullptr;
-  if (op.panels->sell) return op.panels->sell.get();
-  if (op.n <= 0 || op.n >= int64_t(0xffffffff) - kSellSortRows || op.nnz >= (int64_t(1) << 32)) return nullptr;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  SI_CUDA(cudaStreamIsCapturing(ex.stream, &cs));
-  if (cs != cudaStreamCaptureStatusNone) return nullptr;
+// The sliced-ELL copy; null where the memory that it may take does not hold it.
+std::unique_ptr<SellLayout> build_sell(const Exec& ex, const OpDev& op) {
   auto L = std::make_unique<SellLayout>();
   // rows of 4x the mean length or more (at least 128, at most kSellMaxShort+1) are long
   const double mean = static_cast<double>(op.nnz) / static_cast<double>(op.n);
@@ -1363,17 +1361,15 @@ const SellLayout* sell_layout(const Exec& ex, const OpDev& op) {
   L->slice_ptr.alloc(static_cast<size_t>(L->n_slices + 1), ex.stream);
   L->slots = exclusive_scan_u64(ex, cnt.get(), L->slice_ptr.get(), L->n_slices);
   // The copy must fit beside what else the program needs: a prepared operator
-  // has its budget from its creation; a solve, which drops the copy again when
-  // it runs out of memory, asks the driver only for copies of gigabytes
+  // has its budget from its creation; a solve, which goes on without the copy
+  // where memory runs out, now or later, asks the driver only for copies of gigabytes
   // (cudaMemGetInfo was seen to take 30 to 80 ms behind queued frees).
   const size_t per_slot = 4 + (op.v32 ? 4 : 0) + (op.v64 ? 8 : 0);
   const uint64_t want = L->slots * per_slot;
   uint64_t budget = op.panels->sell_budget;
   if (budget == 0 && want > uint64_t(2) << 30) budget = free_memory_quarter();
-  if (budget != 0 && want > budget) {
-    op.panels->sell_failed = true;
-    return nullptr;
-  }
+  if (budget != 0 && want > budget) return nullptr;
+  if (copy_oom_seam("build")) throw Error(SI_OUT_OF_MEMORY, "sliced copy: out of memory (test seam)");
   L->idx.alloc(static_cast<size_t>(std::max<uint64_t>(L->slots, 1)), ex.stream);
   if (op.v32) L->v32.alloc(static_cast<size_t>(std::max<uint64_t>(L->slots, 1)), ex.stream);
   if (op.v64) L->v64.alloc(static_cast<size_t>(std::max<uint64_t>(L->slots, 1)), ex.stream);
@@ -1381,7 +1377,26 @@ const SellLayout* sell_layout(const Exec& ex, const OpDev& op) {
   k_sell_fill<<<g2, 256, 0, ex.stream>>>(L->n_slices, L->slice_ptr.get(), L->perm.get(), L->plen.get(), op.indptr,
                                           op.indices, op.v32, op.v64, L->idx.get(), L->v32.get(), L->v64.get());
   SI_LAUNCH_CHECK();
-  op.panels->sell = std::move(L);
+  return L;
+}
+
+// The operator's sliced copy (built on first use, outside stream capture, for
+// owners that allow it; null when not available).  Products do without it, so
+// memory running out while it is built is no error of theirs.
+const SellLayout* sell_layout(const Exec& ex, const OpDev& op) {
+  if (op.panels == nullptr || !op.panels->sell_ok || op.panels->sell_failed) return nullptr;
+  if (op.panels->sell) return op.panels->sell.get();
+  if (op.n <= 0 || op.n >= int64_t(0xffffffff) - kSellSortRows || op.nnz >= (int64_t(1) << 32)) return nullptr;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  SI_CUDA(cudaStreamIsCapturing(ex.stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return nullptr;
+  try {
+    op.panels->sell = build_sell(ex, op);
+  } catch (const Error& e) {
+    if (e.code != SI_OUT_OF_MEMORY) throw;
+    cudaGetLastError();  // the failed allocation's
+  }
+  op.panels->sell_failed = !op.panels->sell;
   return op.panels->sell.get();
 }
 

@@ -271,3 +271,33 @@ def test_spmm_tuning_file(gpu_ctx, monkeypatch, tmp_path):
     mine = [l for l in lines if int(l[0]) == n and int(l[1]) == a.nnz]
     assert mine and all(len(l) == 9 and int(l[2]) == 4 and int(l[3]) == 8 and int(l[4]) == 8 for l in mine)
     op.close()
+
+
+def test_no_memory_for_the_sliced_copy(gpu_ctx, monkeypatch):
+    """Memory that runs out for the copy itself, or for a solve that holds one
+    (SPECTRAL_INIT_COPY_OOM, a test seam): products and solves go on without
+    it, as the vector kernel alone forms them."""
+    import torch
+    import spectral_init_b200 as si
+    rng = np.random.default_rng(3)
+    n = 110_003  # about 2.4 M entries: above 2^21, where the sliced kernels are the rule
+    a = sp.random(n, n, density=10.0 / n, random_state=rng, format="csr")
+    a = (a + a.T + sp.diags([1.0, 1.0], [1, -1], shape=(n, n))).tocsr()
+    inv = 1.0 / np.sqrt(np.asarray(a.sum(axis=1)).ravel())
+    lap = (sp.identity(n) - sp.diags(inv) @ a @ sp.diags(inv)).tocsr()
+    assert lap.nnz >= 1 << 21
+    x = rng.standard_normal((n, 4))
+    cfg = si.SpectralInitConfig(tol=1e-8)
+    got = {}
+    for seam in ("", "build", "solve"):
+        monkeypatch.setenv("SPECTRAL_INIT_COPY_OOM", seam)
+        op = si.CsrOperator(lap, diag=0.0, ctx=gpu_ctx)
+        y = op.apply_prepared(torch.from_numpy(x).cuda())
+        gpu_ctx.synchronize()
+        assert _rel(y.cpu().numpy(), lap @ x) < 1e-14
+        op.close()
+        (vals, vecs), _ = si.lobpcg_solve(lap, 2, 42, False, 1.0 / inv, cfg, ctx=gpu_ctx)
+        assert np.max(np.linalg.norm(lap @ vecs - vecs * vals, axis=0)) < 1e-7
+        got[seam] = vals, vecs
+    assert all(np.array_equal(p, q) for p, q in zip(got["build"], got["solve"]))
+    assert np.max(np.abs(got[""][0] - got["build"][0])) < 1e-12
