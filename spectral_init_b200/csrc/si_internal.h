@@ -122,7 +122,8 @@ void make_row_blocks(const Exec& ex, const OpDev& op, RowBlocks& rb);
 void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok);
 uint64_t free_memory_quarter();
 // Test seam SPECTRAL_INIT_COPY_OOM: out of memory for the sliced copy itself
-// ("build") or for the solve that holds one ("solve").
+// ("build"), for the solve that holds one ("solve"), or for the padded blocks of
+// a product ("blocks").
 bool copy_oom_seam(const char* where);
 // Build the sliced copy of an attached operator now, where the rule uses it.
 void build_sliced_copy(const Exec& ex, const OpDev& op);

@@ -1720,9 +1720,21 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
     // 86 at n = 300k shuffled, 9 columns 774 / 588 at n = 800k; level at n = 20k)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     SI_CUDA(cudaStreamIsCapturing(ex.stream, &cs));
-    if (cs == cudaStreamCaptureStatusNone) {
-      const int lp = k <= 4 ? 4 : (k <= 8 ? 8 : 16);
-      DevBuf<XT> xp(static_cast<size_t>(op.n) * lp, ex.stream), yp(static_cast<size_t>(op.n) * lp, ex.stream);
+    const int lp = k <= 4 ? 4 : (k <= 8 ? 8 : 16);
+    DevBuf<XT> xp, yp;
+    bool room = cs == cudaStreamCaptureStatusNone;
+    if (room) {
+      try {
+        if (copy_oom_seam("blocks")) throw Error(SI_OUT_OF_MEMORY, "padded blocks: out of memory (test seam)");
+        xp.alloc(static_cast<size_t>(op.n) * lp, ex.stream);
+        yp.alloc(static_cast<size_t>(op.n) * lp, ex.stream);
+      } catch (const Error& e) {  // the generic kernel needs none
+        if (e.code != SI_OUT_OF_MEMORY) throw;
+        cudaGetLastError();
+        room = false;
+      }
+    }
+    if (room) {
       const int g1 = static_cast<int>(std::min<int64_t>((op.n * lp + 255) / 256, int64_t(ex.sms) * 16));
       k_pad_rows<XT><<<g1, 256, 0, ex.stream>>>(op.n, k, x, ld, xp.get(), lp);
       SI_LAUNCH_CHECK();

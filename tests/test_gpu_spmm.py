@@ -301,3 +301,42 @@ def test_no_memory_for_the_sliced_copy(gpu_ctx, monkeypatch):
         got[seam] = vals, vecs
     assert all(np.array_equal(p, q) for p, q in zip(got["build"], got["solve"]))
     assert np.max(np.abs(got[""][0] - got["build"][0])) < 1e-12
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("n", [30_011, 130_003])
+def test_products_of_any_width_and_base(gpu_ctx, monkeypatch, n, prec):
+    """Widths whose rows the vector gathers cannot take, and bases off by one
+    element, above the entries from which such blocks are packed, below and
+    above those of the sliced kernels; once more with no memory for the packed
+    blocks.  What lies around the result stays as it was."""
+    import torch
+    import spectral_init_b200 as si
+    rng = np.random.default_rng(n)
+    a = sp.random(n, n, density=9.0 / n, random_state=rng, format="csr")
+    a = (a + a.T).tocsr()
+    a.sort_indices()
+    assert 3 << 17 <= a.nnz and (a.nnz >= 1 << 21) == (n > 100_000)
+    dtype, tol = (torch.float64, 1e-14) if prec == "f64" else (torch.float32, 2e-6)
+    av = a if prec == "f64" else sp.csr_matrix((a.data.astype(np.float32).astype(np.float64), a.indices, a.indptr),
+                                               shape=a.shape)
+    op = si.CsrOperator(a, diag=0.75, ctx=gpu_ctx, with_f32=prec == "f32")
+    for k in (1, 2, 3, 4, 5, 7, 8, 9, 13, 15, 16, 17):
+        for off in (0, 1):
+            buf = torch.full((n * k + 2,), 7.0, dtype=dtype, device="cuda")
+            x = buf[off:off + n * k].view(n, k)
+            x.copy_(torch.from_numpy(rng.standard_normal((n, k))))
+            xh = x.cpu().numpy().astype(np.float64)
+            want = 0.75 * xh + av @ xh
+            for seam in ("", "blocks"):
+                monkeypatch.setenv("SPECTRAL_INIT_COPY_OOM", seam)
+                out = torch.full((n * k + 2,), 5.0, dtype=dtype, device="cuda")
+                y = out[off:off + n * k].view(n, k)
+                torch.cuda.synchronize()
+                op.apply_prepared(x, y)
+                gpu_ctx.synchronize()
+                assert _rel(y.cpu().numpy(), want) < tol, (k, off, seam)
+                around = torch.cat([out[:off], out[off + n * k:]])
+                assert bool((around == 5.0).all()), (k, off, seam)
+            assert _rel(op.apply(x).cpu().numpy(), want) < tol, (k, off)
+    op.close()
