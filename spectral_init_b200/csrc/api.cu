@@ -3,7 +3,6 @@
 // message for si_last_error(); nothing unwinds across the ABI.
 #include <cuda_runtime.h>
 
-#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -447,14 +446,8 @@ si_status si_operator_plan_create(si_ctx* ctx, const si_operator* op, si_operato
     p->device = ctx->device;
     p->op = op_of(op);
     p->rb.sell_budget = si::free_memory_quarter();
-    if (std::getenv("SPECTRAL_INIT_SPMM_TUNE_FILE") != nullptr) {  // kernels by timing, kept in that file
-      si::make_row_blocks(ex, p->op, p->rb);
-      p->rb.sell_ok = true;
-      p->rb.attach(p->op);
-    } else {
-      si::attach_ruled(ex, p->op, p->rb, true);
-      si::build_sliced_copy(ex, p->op);
-    }
+    si::attach_ruled(ex, p->op, p->rb, true);
+    si::build_sliced_copy(ex, p->op);
     SI_CUDA(cudaStreamSynchronize(ex.stream));
     *out = p.release();
   });

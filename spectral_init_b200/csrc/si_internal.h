@@ -117,15 +117,16 @@ struct RowBlocks {
   }
 };
 void make_row_blocks(const Exec& ex, const OpDev& op, RowBlocks& rb);
-// An operator of one solve (sell_ok: applied many times) or one call: kernels
-// by rule, the partitions above only when a forced kernel may need them.
+// A prepared operator or one of one solve (sell_ok: applied many times), or of
+// one call: kernels by rule, unless SPECTRAL_INIT_SPMM_TUNE_FILE names a file of
+// timed choices; the partitions above only where a kernel may need them.
 void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok);
 uint64_t free_memory_quarter();
 // Test seam SPECTRAL_INIT_COPY_OOM: out of memory for the sliced copy itself
 // ("build"), for the solve that holds one ("solve"), or for the padded blocks of
 // a product ("blocks").
 bool copy_oom_seam(const char* where);
-// Build the sliced copy of an attached operator now, where the rule uses it.
+// Build the sliced copy of an attached operator now, where the rule may use it.
 void build_sliced_copy(const Exec& ex, const OpDev& op);
 
 // Epilogue of an SpMM: out = alpha * (A x) + beta * z1 + gamma * z2 + delta * z3

@@ -1755,19 +1755,18 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
 }  // namespace
 
 void build_sliced_copy(const Exec& ex, const OpDev& op) {
-  if (op.nnz >= kSlicedMinNnz) sell_layout(ex, op);
+  if (op.panels->ruled && op.nnz >= kSlicedMinNnz) sell_layout(ex, op);
 }
 
 void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok) {
+  const bool timed = std::getenv("SPECTRAL_INIT_SPMM_TUNE_FILE") != nullptr;
+  bool forced = false;
   for (const char* name :
-       {"SPECTRAL_INIT_SPMM_KERNEL", "SPECTRAL_INIT_SPMM_KERNEL_F32", "SPECTRAL_INIT_SPMM_KERNEL_F64"}) {
-    if (std::getenv(name) != nullptr) {
-      make_row_blocks(ex, op, rb);
-      break;
-    }
-  }
+       {"SPECTRAL_INIT_SPMM_KERNEL", "SPECTRAL_INIT_SPMM_KERNEL_F32", "SPECTRAL_INIT_SPMM_KERNEL_F64"})
+    forced = forced || std::getenv(name) != nullptr;
+  if (timed || forced) make_row_blocks(ex, op, rb);
   rb.sell_ok = sell_ok;
-  rb.ruled = true;
+  rb.ruled = !timed;
   rb.attach(op);
 }
 

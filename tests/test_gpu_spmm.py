@@ -340,3 +340,23 @@ def test_products_of_any_width_and_base(gpu_ctx, monkeypatch, n, prec):
                 assert bool((around == 5.0).all()), (k, off, seam)
             assert _rel(op.apply(x).cpu().numpy(), want) < tol, (k, off)
     op.close()
+
+
+def test_solve_keeps_its_choices_in_the_tuning_file(gpu_ctx, monkeypatch, tmp_path):
+    """A solve on an operator of 2^22 or more entries times its kernels while a
+    tuning file is named, as a prepared operator does, and appends what it chose."""
+    import spectral_init_b200 as si
+    rng = np.random.default_rng(22)
+    n = 262_151  # a shape no other test uses, about 5 M entries
+    a = sp.random(n, n, density=9.0 / n, random_state=rng, format="csr")
+    a = (a + a.T + sp.diags([1.0, 1.0], [1, -1], shape=(n, n))).tocsr()
+    inv = 1.0 / np.sqrt(np.asarray(a.sum(axis=1)).ravel())
+    lap = (sp.identity(n) - sp.diags(inv) @ a @ sp.diags(inv)).tocsr()
+    path = tmp_path / "tune.txt"
+    monkeypatch.setenv("SPECTRAL_INIT_SPMM_TUNE_FILE", str(path))
+    monkeypatch.delenv("SPECTRAL_INIT_SPMM_KERNEL", raising=False)
+    cfg = si.SpectralInitConfig(tol=1e-6)
+    (vals, vecs), _ = si.lobpcg_solve(lap, 2, 42, False, 1.0 / inv, cfg, ctx=gpu_ctx)
+    assert np.max(np.linalg.norm(lap @ vecs - vecs * vals, axis=0)) < 1e-5
+    lines = [l.split() for l in path.read_text().splitlines()]
+    assert any(int(l[0]) == n and int(l[1]) == lap.nnz and int(l[2]) == 4 for l in lines)
