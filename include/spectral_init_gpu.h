@@ -205,9 +205,10 @@ si_status si_spmm_f32(si_ctx* ctx, const si_operator* op, const float* x, float*
 
 /* A device operator prepared for repeated products (the crate's CsrOperator,
  * src/operator.rs:174-228, holds its matrix across LinearOperator::apply
- * calls): the row partitions of the tiled / gather / panel kernels are built
- * once; the sliced copy of the operator (the kernel of operators of 2^21 or
- * more entries, about the size of the index and value arrays again) with it, the
+ * calls).  The sliced copy of the operator (for most products of operators of
+ * 2^21 or more entries, about the size of the index and value arrays again) is
+ * built with it where 1/64 of the free memory holds the copy, otherwise by the
+ * first product that uses it, outside stream capture, where a quarter does; the
  * panel kernel's x windows on first use, outside stream capture.  The
  * operator's arrays must stay allocated and unchanged while the plan lives,
  * and calls on one plan from several host threads must be serialised by the

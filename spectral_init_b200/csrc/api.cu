@@ -445,7 +445,7 @@ si_status si_operator_plan_create(si_ctx* ctx, const si_operator* op, si_operato
     std::unique_ptr<si_operator_plan> p(new si_operator_plan());
     p->device = ctx->device;
     p->op = op_of(op);
-    p->rb.sell_budget = si::free_memory_quarter();
+    p->rb.sell_outlives = true;
     si::attach_ruled(ex, p->op, p->rb, true);
     si::build_sliced_copy(ex, p->op);
     SI_CUDA(cudaStreamSynchronize(ex.stream));

@@ -102,7 +102,7 @@ struct RowBlocks {
   bool sell_ok = false;
   mutable std::unique_ptr<SellLayout> sell;
   mutable bool sell_failed = false;
-  uint64_t sell_budget = 0;  // most bytes the copy may take (0: not asked for)
+  bool sell_outlives = false;  // the copy is kept after the call that builds it
   // kernels by the rule on shape and types instead of by timing candidates
   // (operators of one solve or one call, whose first pass is what counts)
   bool ruled = false;
@@ -121,12 +121,15 @@ void make_row_blocks(const Exec& ex, const OpDev& op, RowBlocks& rb);
 // one call: kernels by rule, unless SPECTRAL_INIT_SPMM_TUNE_FILE names a file of
 // timed choices; the partitions above only where a kernel may need them.
 void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok);
-uint64_t free_memory_quarter();
+uint64_t free_memory();
 // Test seam SPECTRAL_INIT_COPY_OOM: out of memory for the sliced copy itself
 // ("build"), for the solve that holds one ("solve"), or for the padded blocks of
-// a product ("blocks").
+// a product ("blocks"); 1 GiB of free memory ("tight").
 bool copy_oom_seam(const char* where);
-// Build the sliced copy of an attached operator now, where the rule may use it.
+// Build the sliced copy of an attached operator now, where the rule may use it
+// and at most 1/64 of the free memory holds it: what products come is not known
+// yet (the rule has none of 16 f64 columns on it), so larger copies wait for the
+// first that wants one.
 void build_sliced_copy(const Exec& ex, const OpDev& op);
 
 // Epilogue of an SpMM: out = alpha * (A x) + beta * z1 + gamma * z2 + delta * z3

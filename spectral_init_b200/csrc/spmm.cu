@@ -1321,11 +1321,13 @@ bool copy_oom_seam(const char* where) {
   return v != nullptr && std::string(v) == where;
 }
 
-uint64_t free_memory_quarter() {
+uint64_t free_memory() {
   size_t free_b = 0, total_b = 0;
   SI_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  return std::max<uint64_t>(free_b / 4, 1);
+  return copy_oom_seam("tight") ? std::min<size_t>(free_b, size_t(1) << 30) : free_b;
 }
+
+uint64_t slot_bytes(const OpDev& op) { return 4 + (op.v32 ? 4 : 0) + (op.v64 ? 8 : 0); }
 
 namespace {
 
@@ -1360,15 +1362,12 @@ std::unique_ptr<SellLayout> build_sell(const Exec& ex, const OpDev& op) {
   SI_LAUNCH_CHECK();
   L->slice_ptr.alloc(static_cast<size_t>(L->n_slices + 1), ex.stream);
   L->slots = exclusive_scan_u64(ex, cnt.get(), L->slice_ptr.get(), L->n_slices);
-  // The copy must fit beside what else the program needs: a prepared operator
-  // has its budget from its creation; a solve, which goes on without the copy
-  // where memory runs out, now or later, asks the driver only for copies of gigabytes
+  // The copy must fit beside what else the program needs, a quarter of the free
+  // memory at most; a solve, which goes on without the copy where memory runs
+  // out, now or later, asks the driver only for copies of gigabytes
   // (cudaMemGetInfo was seen to take 30 to 80 ms behind queued frees).
-  const size_t per_slot = 4 + (op.v32 ? 4 : 0) + (op.v64 ? 8 : 0);
-  const uint64_t want = L->slots * per_slot;
-  uint64_t budget = op.panels->sell_budget;
-  if (budget == 0 && want > uint64_t(2) << 30) budget = free_memory_quarter();
-  if (budget != 0 && want > budget) return nullptr;
+  const uint64_t want = L->slots * slot_bytes(op);
+  if ((op.panels->sell_outlives || want > uint64_t(2) << 30) && want > free_memory() / 4) return nullptr;
   if (copy_oom_seam("build")) throw Error(SI_OUT_OF_MEMORY, "sliced copy: out of memory (test seam)");
   L->idx.alloc(static_cast<size_t>(std::max<uint64_t>(L->slots, 1)), ex.stream);
   if (op.v32) L->v32.alloc(static_cast<size_t>(std::max<uint64_t>(L->slots, 1)), ex.stream);
@@ -1377,6 +1376,7 @@ std::unique_ptr<SellLayout> build_sell(const Exec& ex, const OpDev& op) {
   k_sell_fill<<<g2, 256, 0, ex.stream>>>(L->n_slices, L->slice_ptr.get(), L->perm.get(), L->plen.get(), op.indptr,
                                           op.indices, op.v32, op.v64, L->idx.get(), L->v32.get(), L->v64.get());
   SI_LAUNCH_CHECK();
+  if (op.panels->sell_outlives) SI_CUDA(cudaStreamSynchronize(ex.stream));  // later products may use other streams
   return L;
 }
 
@@ -1755,7 +1755,8 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
 }  // namespace
 
 void build_sliced_copy(const Exec& ex, const OpDev& op) {
-  if (op.panels->ruled && op.nnz >= kSlicedMinNnz) sell_layout(ex, op);
+  if (!op.panels->ruled || op.nnz < kSlicedMinNnz) return;
+  if (static_cast<uint64_t>(op.nnz) * slot_bytes(op) <= free_memory() / 64) sell_layout(ex, op);
 }
 
 void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok) {

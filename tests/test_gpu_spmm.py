@@ -360,3 +360,38 @@ def test_solve_keeps_its_choices_in_the_tuning_file(gpu_ctx, monkeypatch, tmp_pa
     assert np.max(np.linalg.norm(lap @ vecs - vecs * vals, axis=0)) < 1e-5
     lines = [l.split() for l in path.read_text().splitlines()]
     assert any(int(l[0]) == n and int(l[1]) == lap.nnz and int(l[2]) == 4 for l in lines)
+
+
+def test_a_plan_holds_the_copies_that_it_uses(gpu_ctx, monkeypatch):
+    """With little free memory (1 GiB, by a test seam) a prepared operator's
+    sliced copy waits for the first product that the rule gives it: 16 f64
+    columns leave it unbuilt, 4 build it, and destroying the plan frees it."""
+    import torch
+    from cuda.bindings import driver
+    import spectral_init_b200 as si
+
+    def used():
+        gpu_ctx.synchronize()
+        torch.cuda.synchronize()
+        pool = driver.cuDeviceGetDefaultMemPool(0)[1]
+        return int(driver.cuMemPoolGetAttribute(pool, driver.CUmemPool_attribute.CU_MEMPOOL_ATTR_USED_MEM_CURRENT)[1])
+
+    monkeypatch.setenv("SPECTRAL_INIT_COPY_OOM", "tight")
+    rng = np.random.default_rng(5)
+    n = 150_001
+    a = sp.random(n, n, density=8.0 / n, random_state=rng, format="csr")
+    a = (a + a.T).tocsr()
+    a.sort_indices()
+    copy = 12 * a.nnz  # indices and f64 values
+    assert a.nnz >= 1 << 21 and (1 << 30) // 64 < copy < (1 << 30) // 4
+    op = si.CsrOperator(a, diag=1.0, ctx=gpu_ctx)
+    base = used()
+    op.prepare()
+    blocks = {k: rng.standard_normal((n, k)) for k in (16, 4)}
+    for k, x in blocks.items():
+        y = op.apply_prepared(torch.from_numpy(x).cuda())
+        gpu_ctx.synchronize()
+        assert _rel(y.cpu().numpy(), x + a @ x) < 1e-14
+        assert (used() - base >= copy) == (k == 4)
+    op.close()
+    assert used() <= base
