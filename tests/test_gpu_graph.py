@@ -123,3 +123,31 @@ def test_invalid_graphs_are_rejected(gpu_ctx, bad):
         data[0] = np.nan
     with pytest.raises(si.InvalidGraph):
         si.spectral_init((indptr, indices, data, 3), 1, 42, ctx=gpu_ctx)
+
+
+@pytest.mark.parametrize("kind", ["path", "band", "ladder", "ladders"])
+def test_components_of_long_chains(gpu_ctx, kind):
+    """Graphs whose roots hook into chains as long as the graph: a path and a
+    band of nodes in order, and rungs a_i - b_i - c_i whose b_i are joined by
+    edges that are neither first nor last in their rows; once as one graph and
+    once cut into 500.  Every node gets its component's number."""
+    import spectral_init_b200 as si
+    m = 200_003
+    i = np.arange(m - 1)
+    if kind == "path":
+        r, c = i, i + 1
+    elif kind == "band":
+        r, c = np.concatenate([i[:m - d] for d in range(1, 9)]), np.concatenate([i[:m - d] + d for d in range(1, 9)])
+        r, c = r[c < m], c[c < m]
+    else:
+        a = np.arange(m)
+        keep = i if kind == "ladder" else i[(i + 1) % 401 != 0]
+        r, c = np.r_[a, a + 2 * m, keep + m], np.r_[a + m, a + m, keep + m + 1]
+    n = m if kind in ("path", "band") else 3 * m
+    g = sp.coo_matrix((np.ones(2 * r.size, np.float32), (np.r_[r, c], np.r_[c, r])), shape=(n, n)).tocsr()
+    g.sort_indices()
+    nc, want = sp.csgraph.connected_components(g, directed=False)
+    for _ in range(3):
+        labels, got = si.find_components(g, ctx=gpu_ctx)
+        assert got == nc
+        assert np.array_equal(labels, want)
