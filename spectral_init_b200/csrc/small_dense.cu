@@ -129,6 +129,30 @@ __device__ double cta_sum(double v, double* red) {
   return t;
 }
 
+// Scales a finite A by a power of two (exact) to a largest entry in [1, 2): the
+// Jacobi iteration below forms its angles in single precision and sums squares.
+// Returns the factor that takes eigenvalues back, zero where A is not finite.  A
+// function of its own: part of the iteration, it cost the direct route's callers
+// 2.4 us a step of 48 columns.
+__device__ __noinline__ double cta_unit_scale(double* A, int s, int ld, double* red) {
+  double big = 0.0;
+  int bad = 0;
+  for (int t = threadIdx.x; t < s * s; t += blockDim.x) {
+    const double a = fabs(A[(t / s) * ld + t % s]);
+    big = fmax(big, a);
+    if (!(a <= DBL_MAX)) bad = 1;
+  }
+  big = warp_max(big);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = big;
+  if (__syncthreads_or(bad)) return 0.0;
+  for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) big = fmax(big, red[i]);
+  const int ex = min(max(__double2hiint(big) >> 20, 1), 2045);  // exponent field
+  const double sc = __hiloint2double((2046 - ex) << 20, 0);
+  for (int t = threadIdx.x; t < s * s; t += blockDim.x) A[(t / s) * ld + t % s] *= sc;
+  __syncthreads();
+  return __hiloint2double(ex << 20, 0);
+}
+
 // Parallel cyclic Jacobi with one update phase per round: the round's
 // disjoint rotations J are applied as A' = J^T A J and V' = V J in a single
 // pass into second buffers (every element of A' depends on a 2 x 2 block of
@@ -141,11 +165,9 @@ __device__ double cta_sum(double v, double* red) {
 // A and V stay exactly similar / orthogonal, and an angle off by ~1e-7 only
 // leaves ~1e-7 of a_pq for the next sweep (quadratic convergence down to that
 // level, then a factor ~1e-7 per sweep).  No f64 square root or division on
-// the round's critical path.  The single-precision angle and the sums of
-// squares want entries of order one: A is scaled by a power of two (exact)
-// first.  On return A's diagonal and V hold the result; false, with nothing
-// done, where A is not finite.
-__device__ bool cta_jacobi_db(double* A, double* V, double* A2, double* V2, int s, int ld, double* red) {
+// the round's critical path.  On return A (diagonal) and V hold the result.
+// Wants finite entries of order one (cta_unit_scale).
+__device__ void cta_jacobi_db(double* A, double* V, double* A2, double* V2, int s, int ld, double* red) {
   __shared__ double al[3 * MAXM + 2], be[3 * MAXM + 2];
   __shared__ int pq[3 * MAXM + 2];
   constexpr int kItems = 9;  // per-thread update items resolved once when 2 s^2 <= 9 * threads
@@ -161,25 +183,6 @@ __device__ bool cta_jacobi_db(double* A, double* V, double* A2, double* V2, int 
     it_i[q] = u / s;
     it_j[q] = u - (u / s) * s;
   }
-  double big = 0.0;
-  int bad = 0;
-  for (int t = threadIdx.x; t < s * s; t += blockDim.x) {
-    const int i = t / s, j = t - (t / s) * s;
-    const double a = fabs(A[i * ld + j]);
-    big = fmax(big, a);
-    if (!(a <= DBL_MAX)) bad = 1;
-  }
-  big = warp_max(big);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = big;
-  if (__syncthreads_or(bad)) return false;
-  for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) big = fmax(big, red[i]);
-  const int ex = min(max(__double2hiint(big) >> 20, 1), 2045);  // exponent field
-  const double sc = __hiloint2double((2046 - ex) << 20, 0), unscale = __hiloint2double(ex << 20, 0);
-  for (int t = threadIdx.x; t < s * s; t += blockDim.x) {
-    const int i = t / s, j = t - (t / s) * s;
-    A[i * ld + j] *= sc;
-  }
-  __syncthreads();
   double* cur = A;
   double* nxt = A2;
   double* vc = V;
@@ -275,11 +278,8 @@ __device__ bool cta_jacobi_db(double* A, double* V, double* A2, double* V2, int 
       A[i * ld + j] = cur[i * ld + j];
       V[i * ld + j] = vc[i * ld + j];
     }
-    __syncthreads();
   }
-  for (int i = threadIdx.x; i < s; i += blockDim.x) A[i * ld + i] *= unscale;
   __syncthreads();
-  return true;
 }
 
 // Parallel cyclic Jacobi (round-robin pairing): A <- diag, V <- eigenvectors
@@ -504,11 +504,10 @@ __device__ bool cta_rr_general(const double* gb, const double* ga, int P, const 
   __syncthreads();
   cta_identity(sm.V, s, ld);
   __syncthreads();
-  if (s <= 3 * MAXM) {
-    if (!cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red)) return false;
-  } else {
-    cta_jacobi(sm.A, sm.V, s, ld, red, rc, rs, ra, rb);
-  }
+  const double unscale = cta_unit_scale(sm.A, s, ld, red);
+  if (unscale == 0.0) return false;
+  if (s <= 3 * MAXM) cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red);
+  else cta_jacobi(sm.A, sm.V, s, ld, red, rc, rs, ra, rb);
   if (threadIdx.x == 0) {
     sort_eigs(sm.A, s, ld, order);
     if (largest) {
@@ -518,7 +517,7 @@ __device__ bool cta_rr_general(const double* gb, const double* ga, int P, const 
         order[s - 1 - i] = t;
       }
     }
-    for (int q = 0; q < nsel; ++q) theta_out[q] = sm.A[order[q] * ld + order[q]];
+    for (int q = 0; q < nsel; ++q) theta_out[q] = sm.A[order[q] * ld + order[q]] * unscale;
   }
   __syncthreads();
   // Z = V[:, order[0..nsel)]
@@ -1133,7 +1132,6 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
     if (lane == 0) sscale = fit ? __hiloint2double((1023 + ex) << 20, 0) : 0.0;
   }
   __syncthreads();
-  if (sscale == 0.0) return false;
   // ---- eigenvalues and vectors, one warp each ----
   double2* Lp = reinterpret_cast<double2*>(work) + warp * 2 * kTriMax;  // per warp: two rows
   for (int q = warp; q < nsel; q += nw) {
@@ -1282,7 +1280,7 @@ __device__ bool cta_tri_select(double* A, int s, int ld, int nsel, int largest, 
   }
   // ---- residual test in the tridiagonal basis, at what Jacobi ends with (750
   // steps of solves at 1e-10, widths 4 to 48: at most 0.7 eps) ----
-  int off = fine ? 0 : 1;
+  int off = fine && sscale != 0.0 ? 0 : 1;
   for (int t = threadIdx.x; t < s * nsel; t += nt) {
     const int i = t / nsel, q = t - (t / nsel) * nsel;
     double r = (d[i] - th[q]) * V[i * ld + q];
@@ -1377,6 +1375,47 @@ __device__ bool cta_inverse_cholesky(double* B, int s, int ld, double tol, doubl
     if (lane < s) B[i * ld + lane] = lane < i ? a0[q] * f : (lane == i ? f : 0.0);
     if (WIDE && l1 < s) B[i * ld + l1] = l1 < i ? a1[q] * f : (l1 == i ? f : 0.0);
   }
+  return true;
+}
+
+// The nsel smallest (largest) eigenpairs of sm.A by the Jacobi iteration over all:
+// theta_out the values, order their columns of sm.V.  False where A is not finite.
+// Not inlined: it is the rare branch of a kernel that spills.
+__device__ __noinline__ bool cta_jacobi_pairs(SmallSmem sm, int s, int nsel, int largest, double* theta_out, double* red,
+                                              int* order) {
+  const int ld = sm.ld, nt = blockDim.x;
+  cta_identity(sm.V, s, ld);
+  for (int t = threadIdx.x; t < s * s; t += nt) {  // C to exact symmetry
+    const int i = t / s, j = t - (t / s) * s;
+    if (j > i) sm.T[i * ld + j] = 0.5 * (sm.A[i * ld + j] + sm.A[j * ld + i]);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < s * s; t += nt) {
+    const int i = t / s, j = t - (t / s) * s;
+    if (j > i) {
+      sm.A[i * ld + j] = sm.T[i * ld + j];
+      sm.A[j * ld + i] = sm.T[i * ld + j];
+    }
+  }
+  __syncthreads();
+  const double unscale = cta_unit_scale(sm.A, s, ld, red);
+  if (unscale == 0.0) return false;  // no order: the ranks below would not cover it
+  cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red);
+  // ---- selection by ranks (ascending, or descending for `largest`; ties by index) ----
+  for (int i = threadIdx.x; i < s; i += nt) {
+    const double di = sm.A[i * ld + i];
+    int rank = 0;
+    for (int j = 0; j < s; ++j) {
+      const double dj = sm.A[j * ld + j];
+      // ascending and stable; for `largest` the reverse of that order
+      const bool before = largest ? (dj > di || (dj == di && j > i)) : (dj < di || (dj == di && j < i));
+      rank += before ? 1 : 0;
+    }
+    order[rank] = i;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < nsel; q += nt) theta_out[q] = sm.A[order[q] * ld + order[q]] * unscale;
+  __syncthreads();
   return true;
 }
 
@@ -1498,36 +1537,7 @@ __device__ bool cta_rr_general_par(const double* gb, const double* ga, int P, co
     for (int q = threadIdx.x; q < nsel; q += nt) order[q] = q;
     __syncthreads();
   } else {
-    cta_identity(sm.V, s, ld);
-    for (int t = threadIdx.x; t < s * s; t += nt) {  // C to exact symmetry
-      const int i = t / s, j = t - (t / s) * s;
-      if (j > i) sm.T[i * ld + j] = 0.5 * (sm.A[i * ld + j] + sm.A[j * ld + i]);
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < s * s; t += nt) {
-      const int i = t / s, j = t - (t / s) * s;
-      if (j > i) {
-        sm.A[i * ld + j] = sm.T[i * ld + j];
-        sm.A[j * ld + i] = sm.T[i * ld + j];
-      }
-    }
-    __syncthreads();
-    // (a C that is not finite has no order: the ranks below would not cover it)
-    if (!cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, s, ld, red)) return false;
-    // ---- selection by ranks (ascending, or descending for `largest`; ties by index) ----
-    for (int i = threadIdx.x; i < s; i += nt) {
-      const double di = sm.A[i * ld + i];
-      int rank = 0;
-      for (int j = 0; j < s; ++j) {
-        const double dj = sm.A[j * ld + j];
-        // ascending and stable; for `largest` the reverse of that order
-        const bool before = largest ? (dj > di || (dj == di && j > i)) : (dj < di || (dj == di && j < i));
-        rank += before ? 1 : 0;
-      }
-      order[rank] = i;
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < nsel; q += nt) theta_out[q] = sm.A[order[q] * ld + order[q]];
+    if (!cta_jacobi_pairs(sm, s, nsel, largest, theta_out, red, order)) return false;
   }
   // ---- Z = D M^T V_sel ----
   for (int t = threadIdx.x; t < s * nsel; t += nt) {
@@ -1638,10 +1648,11 @@ __device__ void small_step_body(LobpcgCtrl* ctrl, LobpcgCtrl* gctrl, const doubl
     __syncthreads();
     cta_identity(sm.V, m, LDS);
     __syncthreads();
-    cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, m, LDS, red);
+    const double unscale = cta_unit_scale(sm.A, m, LDS, red);
+    if (unscale != 0.0) cta_jacobi_db(sm.A, sm.V, sm.T, sm.Z, m, LDS, red);
     if (threadIdx.x == 0) {
       sort_eigs(sm.A, m, LDS, order);
-      for (int q = 0; q < m; ++q) ctrl->lam[q] = sm.A[order[q] * LDS + order[q]];
+      for (int q = 0; q < m; ++q) ctrl->lam[q] = sm.A[order[q] * LDS + order[q]] * (unscale != 0.0 ? unscale : 1.0);
     }
     __syncthreads();
     for (int t = threadIdx.x; t < MAXM * MAXM; t += blockDim.x) {
