@@ -106,6 +106,7 @@ struct RowBlocks {
   // kernels by the rule on shape and types instead of by timing candidates
   // (operators of one solve or one call, whose first pass is what counts)
   bool ruled = false;
+  int64_t longest = -1;  // entries of the longest row (-1: not looked for)
   void attach(OpDev& op) const {
     op.row_blocks = starts.get();
     op.block_ptr = ptrs.get();

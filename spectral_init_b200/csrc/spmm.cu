@@ -1500,7 +1500,40 @@ struct TuneKey {
 std::mutex g_tune_mu;
 std::map<TuneKey, int> g_tune;
 constexpr int64_t kTuneMinNnz = int64_t(1) << 22;  // operators the autotuner times
-constexpr int64_t kSlicedMinNnz = int64_t(1) << 21;  // operators whose rule asks for the sliced kernels
+constexpr int64_t kSlicedMinNnz = int64_t(1) << 21;  // operators whose rule may ask for the sliced kernels
+constexpr int64_t kLongestMinNnz = int64_t(1) << 18;  // operators whose longest row is looked for
+
+double mean_row(const OpDev& op) { return op.n > 0 ? static_cast<double>(op.nnz) / static_cast<double>(op.n) : 0.0; }
+
+// Rows of about one length: at most what a Poisson distribution of the mean
+// reaches (neighbour graphs reach twenty to forty times the mean).
+bool even_rows(const OpDev& op) {
+  return op.panels != nullptr && op.panels->longest >= 0 &&
+         static_cast<double>(op.panels->longest) <= 4.0 * mean_row(op) + 16.0;
+}
+
+__global__ void __launch_bounds__(256) k_longest_row(int64_t n, const uint64_t* __restrict__ indptr,
+                                                     unsigned long long* __restrict__ out) {
+  unsigned long long m = 0;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
+    m = max(m, static_cast<unsigned long long>(indptr[i + 1] - indptr[i]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0 && m != 0) atomicMax(out, m);
+}
+
+int64_t longest_row(const Exec& ex, const OpDev& op) {
+  DevBuf<unsigned long long> out(1, ex.stream);
+  out.zero();
+  const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((op.n + 255) / 256, int64_t(ex.sms) * 8)));
+  k_longest_row<<<grid, 256, 0, ex.stream>>>(op.n, op.indptr, out.get());
+  SI_LAUNCH_CHECK();
+  unsigned long long h = 0;
+  SI_CUDA(cudaMemcpyAsync(&h, out.get(), sizeof(h), cudaMemcpyDeviceToHost, ex.stream));
+  SI_CUDA(cudaStreamSynchronize(ex.stream));
+  return static_cast<int64_t>(h);
+}
 
 // Tuning file (SPECTRAL_INIT_SPMM_TUNE_FILE): choices keyed by the operator's
 // shape rather than its addresses, one line "n nnz ld vbytes xbytes tiled
@@ -1586,17 +1619,32 @@ int forced_choice(const OpDev& op, bool tiled) {
 // M, 312 / 354 at n = 1M; 16 columns, f32: 140 / 97 and 480 / 541), and 16 f64
 // columns gain nothing clear (780 / 710 in cluster order, 805 / 827 shuffled;
 // four passes of four columns: 1051 and 1182).
-template <class VT, class XT, int LD>
-int ruled_choice(const OpDev& op) {
+//
+// Those are neighbour graphs, whose hubs hold tens of times the mean.  Rows of
+// even length (a mesh, a uniform random operator) keep the vector kernel's groups
+// busy: sliced against vector, f64 / f32, 4 columns, 32 / 25 and 28 / 23 with 3 M
+// entries, 36 / 37 and 31 / 35 with 6 M, 138 / 148 and 121 / 126 with 24 M; 20 / 17
+// with 2.4 M entries in 20 000 rows, too few slices for the GPU; wider rows 4 to
+// 40 % behind at every size.  And a few rows beyond a hub's length hold a group
+// of lanes longest (300 000 rows of 15 entries, 50 of 2000, vector against sliced:
+// 146 / 70 and 131 / 54 with 8 columns, 188 / 161 and 189 / 107 with 16).
+int sliced_choice(const OpDev& op, int ld, bool f64) {
+  if (!op.panels->sell_ok || op.nnz < kSlicedMinNnz) return 0;
   const bool large = op.n >= int64_t(1) << 19;
-  if (op.panels->sell_ok && op.nnz >= kSlicedMinNnz) {
-    if (LD == 4) return large ? 402 : 403;
-    if (large) {
-      if (std::is_same<XT, float>::value) return 403;
-      if (LD == 8) return 401;
-    }
+  if (even_rows(op)) {
+    const int64_t from = f64 ? int64_t(11) << 19 : int64_t(9) << 19;
+    return ld == 4 && op.n >= int64_t(1) << 16 && op.nnz >= from ? (large ? 402 : 403) : 0;
   }
-  return spmm_group_lanes(op, LD, sizeof(XT) == 8);
+  if (ld == 4) return large ? 402 : 403;
+  if (static_cast<double>(op.panels->longest) > 64.0 * mean_row(op)) return 403;
+  if (large && !f64) return 403;
+  if (large && ld == 8) return 401;
+  return 0;
+}
+
+int ruled_choice(const OpDev& op, int ld, bool f64) {
+  const int sliced = sliced_choice(op, ld, f64);
+  return sliced != 0 ? sliced : spmm_group_lanes(op, ld, f64);
 }
 
 // Blocks whose row stride or alignment the vector gathers cannot take: packed
@@ -1624,7 +1672,24 @@ __global__ void k_unpad_rows(int64_t n, int k, const XT* __restrict__ in, int ld
   }
 }
 
-constexpr int64_t kPadMinNnz = int64_t(3) << 17;
+// The scalar gathers of the generic kernel cost a request per column and entry,
+// the packing a pass over two blocks (us, generic against packed, neighbour
+// graphs, f64 and f32).  Up to 3 columns fetch a row of 4 either way: 1 column 38 /
+// 46 and 32 / 46 with 2.4 M entries, 93 / 80 and 70 / 75 (shuffled; 62 in cluster
+// order) with 6.2 M, 204 / 130 and 142 / 105 with 20 M; 3 columns 47 / 47 and 37 / 47 with
+// 2.4 M, 71 / 52 and 52 / 45 with 3.6 M.  5 and 9 columns: 48 / 35 and 69 / 56 with 0.9 M
+// (f32 32 / 31, 47 / 49), 411 / 248 and 632 / 435 with 20 M.  Even rows cost the generic
+// kernel less: 1 column 122 / 141 with 24 M entries near the diagonal, 167 / 240
+// with 3 entries a row, 126 / 110 with 200; 3 columns 65 / 48 with 60; 5 columns 48 / 33
+// with 15 entries in 100 000 rows, 135 / 161 with 5 in 1 M.
+bool packing_pays(const OpDev& op, int k) {
+  const double mean = mean_row(op);
+  if (k <= 4) {
+    if (even_rows(op)) return k > 1 && op.nnz >= int64_t(3) << 20 && op.n >= int64_t(1) << 16 && mean >= 48.0;
+    return op.nnz >= (k == 1 ? int64_t(1) << 22 : int64_t(3) << 20) && mean >= 12.0;
+  }
+  return even_rows(op) ? op.nnz >= int64_t(1) << 20 && mean >= 10.0 : op.nnz >= int64_t(3) << 17;
+}
 
 template <class VT, class XT, int LD>
 void dispatch_g(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* y, const Epilogue<XT>& ep,
@@ -1635,7 +1700,7 @@ void dispatch_g(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT
   const TuneKey key{ex.device, op.indptr, op.indices, op.n, op.nnz, LD, static_cast<int>(sizeof(VT)),
                     static_cast<int>(sizeof(XT)), tiled ? 1 : 0, panel ? 1 : 0, sell ? 1 : 0};
   int g = forced_choice<VT, XT, LD>(op, tiled);
-  if (g == 0 && op.panels != nullptr && op.panels->ruled) g = ruled_choice<VT, XT, LD>(op);
+  if (g == 0 && op.panels != nullptr && op.panels->ruled) g = ruled_choice(op, LD, sizeof(XT) == 8);
   if (g != 0) {
     launch_lanes<VT, XT, LD>(g, ex, op, vals, x, y, ep, stop);
     return;
@@ -1714,10 +1779,7 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
   if (aligned && ld == 4) return dispatch_g<VT, XT, 4>(ex, op, vals, x, y, ep, stop);
   if (aligned && ld == 8) return dispatch_g<VT, XT, 8>(ex, op, vals, x, y, ep, stop);
   if (aligned && ld == 16) return dispatch_g<VT, XT, 16>(ex, op, vals, x, y, ep, stop);
-  if (k <= 16 && op.nnz >= kPadMinNnz && ep.z1 == nullptr && ep.z2 == nullptr && ep.z3 == nullptr && stop == nullptr) {
-    // the scalar gathers of the generic kernel cost a request per column and
-    // entry (us, generic against this, f64: 1 column 113 / 84 and 3 columns 129 /
-    // 86 at n = 300k shuffled, 9 columns 774 / 588 at n = 800k; level at n = 20k)
+  if (k <= 16 && packing_pays(op, k) && ep.z1 == nullptr && ep.z2 == nullptr && ep.z3 == nullptr && stop == nullptr) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     SI_CUDA(cudaStreamIsCapturing(ex.stream, &cs));
     const int lp = k <= 4 ? 4 : (k <= 8 ? 8 : 16);
@@ -1744,7 +1806,7 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
       return;
     }
   }
-  switch (spmm_group_lanes(op, 4, sizeof(XT) == 8)) {
+  switch (spmm_group_lanes(op, 0, sizeof(XT) == 8)) {
     case 4: return launch_generic<VT, XT, 4>(ex, op, vals, x, y, ld, k, ep, stop);
     case 8: return launch_generic<VT, XT, 8>(ex, op, vals, x, y, ld, k, ep, stop);
     case 16: return launch_generic<VT, XT, 16>(ex, op, vals, x, y, ld, k, ep, stop);
@@ -1755,7 +1817,7 @@ void dispatch(const Exec& ex, const OpDev& op, const VT* vals, const XT* x, XT* 
 }  // namespace
 
 void build_sliced_copy(const Exec& ex, const OpDev& op) {
-  if (!op.panels->ruled || op.nnz < kSlicedMinNnz) return;
+  if (!op.panels->ruled || (sliced_choice(op, 4, false) == 0 && sliced_choice(op, 4, true) == 0)) return;
   if (static_cast<uint64_t>(op.nnz) * slot_bytes(op) <= free_memory() / 64) sell_layout(ex, op);
 }
 
@@ -1768,6 +1830,7 @@ void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok) {
   if (timed || forced) make_row_blocks(ex, op, rb);
   rb.sell_ok = sell_ok;
   rb.ruled = !timed;
+  if (op.nnz >= kLongestMinNnz) rb.longest = longest_row(ex, op);
   rb.attach(op);
 }
 
@@ -1800,13 +1863,22 @@ int spmm_group_lanes(const OpDev& op, int ld, bool f64) {
   // 40 000: 61 / 46 / 27 / 31 in f32, 72 / 62 / 40 / 26 in f64).  8 and 16
   // columns leave a lane enough columns to reduce only from 16 lanes on, but for
   // 16 f64 columns of many rows (n = 100 000, k = 30: 123 / 135 with 8 / 16 lanes;
-  // 400 000, k = 15: 237 / 277).
-  const double mean = op.n > 0 ? static_cast<double>(op.nnz) / static_cast<double>(op.n) : 0.0;
+  // 400 000, k = 15: 237 / 277) and f32 ones of short rows (400 000, k = 10: 163 / 175).
+  // The generic kernel (ld 0) is full sooner: 36 / 32 and 45 / 39 us with 16 / 8 lanes
+  // (150 000, k = 10, f32, 1 and 3 columns).
+  // Rows of even length end together, and a group of few lanes takes them all
+  // (8 / 16 columns, f32, lanes 4 / 8 / 16: 300 000 rows of 10 35 / 49 / 59 and 53 / 71 /
+  // 102; 20 000 of 120 22 / 20 / 18 and 41 / 34 / 32; f64: 43 / 45 / 67 and 74 / 88 / 113; 33
+  // / 35 / 27 and 60 / 48 / 48; 100 000 of 60 65 / 62 / 64 and 117 / 106 / 108).
+  const double mean = mean_row(op);
+  if (even_rows(op)) return mean <= 28.0 ? 4 : (mean <= 64.0 ? 8 : (mean <= 256.0 ? 16 : 32));
   int g = mean <= 28.0 ? 4 : (mean <= 56.0 ? 8 : (mean <= 112.0 ? 16 : 32));
-  if (ld >= 8) {
-    g = std::max(g, ld == 16 && f64 && op.n >= int64_t(1) << 16 ? 8 : 16);
+  if (ld == 8 || ld == 16) {
+    const bool few = ld == 16 && op.n >= int64_t(1) << 16 && (f64 || mean <= 20.0);
+    g = std::max(g, few ? 8 : 16);
   } else if (mean > 12.0) {
-    while (g < 16 && op.n * g < int64_t(1) << 21) g *= 2;
+    const int64_t full = int64_t(1) << (ld == 4 ? 21 : 20);
+    while (g < 16 && op.n * g < full) g *= 2;
     if (f64 && op.n < int64_t(1) << 16) g = 32;
   }
   while (g < 32 && op.n * g < int64_t(1) << 19) g *= 2;

@@ -273,6 +273,13 @@ def test_spmm_tuning_file(gpu_ctx, monkeypatch, tmp_path):
     op.close()
 
 
+def _hubs(n, rng, count, length):
+    """Symmetric pattern of `count` rows of `length` entries, as a neighbour graph's hubs."""
+    rows = np.repeat(rng.choice(n, count, replace=False), length)
+    h = sp.coo_matrix((rng.uniform(0.1, 1.0, rows.size), (rows, rng.integers(0, n, rows.size))), shape=(n, n))
+    return (h + h.T).tocsr()
+
+
 def test_no_memory_for_the_sliced_copy(gpu_ctx, monkeypatch):
     """Memory that runs out for the copy itself, or for a solve that holds one
     (SPECTRAL_INIT_COPY_OOM, a test seam): products and solves go on without
@@ -282,7 +289,7 @@ def test_no_memory_for_the_sliced_copy(gpu_ctx, monkeypatch):
     rng = np.random.default_rng(3)
     n = 110_003  # about 2.4 M entries: above 2^21, where the sliced kernels are the rule
     a = sp.random(n, n, density=10.0 / n, random_state=rng, format="csr")
-    a = (a + a.T + sp.diags([1.0, 1.0], [1, -1], shape=(n, n))).tocsr()
+    a = (a + a.T + sp.diags([1.0, 1.0], [1, -1], shape=(n, n)) + _hubs(n, rng, 20, 900)).tocsr()
     inv = 1.0 / np.sqrt(np.asarray(a.sum(axis=1)).ravel())
     lap = (sp.identity(n) - sp.diags(inv) @ a @ sp.diags(inv)).tocsr()
     assert lap.nnz >= 1 << 21
@@ -380,7 +387,7 @@ def test_a_plan_holds_the_copies_that_it_uses(gpu_ctx, monkeypatch):
     rng = np.random.default_rng(5)
     n = 150_001
     a = sp.random(n, n, density=8.0 / n, random_state=rng, format="csr")
-    a = (a + a.T).tocsr()
+    a = (a + a.T + _hubs(n, rng, 20, 600)).tocsr()
     a.sort_indices()
     copy = 12 * a.nnz  # indices and f64 values
     assert a.nnz >= 1 << 21 and (1 << 30) // 64 < copy < (1 << 30) // 4
@@ -395,3 +402,33 @@ def test_a_plan_holds_the_copies_that_it_uses(gpu_ctx, monkeypatch):
         assert (used() - base >= copy) == (k == 4)
     op.close()
     assert used() <= base
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("hub", [0, 600, 3000])
+def test_products_with_rows_of_any_spread(gpu_ctx, hub, prec):
+    """Rows of even length, a neighbour graph's hubs and rows far beyond them,
+    which the rules tell apart, against scipy: the packed widths from 2^22
+    entries on and the widths that need no packing."""
+    import torch
+    import spectral_init_b200 as si
+    rng = np.random.default_rng(hub + 1)
+    n = 290_003
+    a = sp.random(n, n, density=7.6 / n, random_state=rng, format="csr")
+    a = (a + a.T + (_hubs(n, rng, 60, hub) if hub else sp.csr_matrix((n, n)))).tocsr()
+    a.sort_indices()
+    longest = int(np.diff(a.indptr).max())
+    assert a.nnz >= 1 << 22 and (longest <= 4 * a.nnz / n + 16) == (hub == 0) and (longest > 64 * a.nnz / n) == (hub == 3000)
+    dtype, tol = (torch.float64, 1e-14) if prec == "f64" else (torch.float32, 2e-6)
+    if prec == "f32":
+        a.data = a.data.astype(np.float32).astype(np.float64)
+    op = si.CsrOperator(a, diag=0.5, ctx=gpu_ctx, with_f32=prec == "f32")
+    for k in (1, 2, 3, 4, 6, 8, 12, 16):
+        x = torch.from_numpy(rng.standard_normal((n, k))).to(device="cuda", dtype=dtype)
+        xh = x.cpu().numpy().astype(np.float64)
+        y = op.apply_prepared(x)
+        gpu_ctx.synchronize()
+        want = 0.5 * xh + a @ xh
+        assert _rel(y.cpu().numpy(), want) < tol, k
+        assert _rel(op.apply(x).cpu().numpy(), want) < tol, k
+    op.close()
