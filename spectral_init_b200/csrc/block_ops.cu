@@ -255,11 +255,13 @@ __global__ void __launch_bounds__(G4_THREADS) k_gram4(const XT* __restrict__ X, 
 // give every product of the two upper triangles in four instructions:
 //   f0 f0: XX XR RR;  f0 f1: XP RP X.AP R.AP;  f0 f2: X.AX X.AR R.AR;
 //   f1 f1: PP P.AP.
-// HBM is the bound (6 n ld s bytes).  The products used to be scalar, four
+// Bytes (6 n ld s) and their latency are the bound.  The products used to be scalar, four
 // warps re-reading a 128-row tile from shared memory (60 reads a row): 48 us
 // f64 and 37 us f32 at n = 1M, 13.5 / 7.2 at n = 200k / 60k, against 27 and 39,
-// 6.3 / 3.9 here (floor 30 and 15 us at n = 1M; f32 is held by the instruction's
-// rate and the conversions, one unit for both).
+// 6.3 / 3.9 here (floor 30 and 15 us at n = 1M; at n = 400k f64 runs at 50 % of
+// HBM, f32 at 20 %, waiting for its 4-byte loads with the matrix pipe at 30 %).
+// The reduction has fewer partials to add: with it f32 at n = 1M takes 55.6 us
+// (48.2 + 7.4, cold caches) where the scalar form took 56.4 (44.4 + 12.0).
 constexpr int GM_THREADS = 256;
 constexpr int GM_UNROLL = 4;  // groups of four rows in flight per warp
 

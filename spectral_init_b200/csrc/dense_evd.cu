@@ -6,16 +6,20 @@
 //      with the matrix spread over the shared memory of co-resident CTAs (a
 //      cluster up to 512 rows, a cooperative launch up to 2048), and three
 //      launches per column above that;
-//   3. split T where off-diagonals are negligible, then for every block the
-//      smallest eigenvalues by Sturm-count multisection (bisection when there
-//      are many blocks) to LAPACK dstebz's default tolerance eps |T|; the k
-//      smallest overall are kept;
-//   4. eigenvectors of T by inverse iteration restricted to the block (LU with
-//      partial pivoting of T - lambda I), re-orthogonalised within clusters of
-//      close eigenvalues (modified Gram-Schmidt), stopped as LAPACK's dstein
-//      once the growth shows a rounding-level residual;
-//   5. back-transformation v = Q y with the stored reflectors (compact-WY
-//      blocks of eight when Y and a block fit in shared memory).
+//   3. up to 2048 rows the k smallest pairs of T directly, a CTA each:
+//      Sturm-count multisection and a twisted factorisation, then one CTA
+//      orthonormalises and tests the vectors;
+//   4. where that test fails (pairs that agree to rounding, a T that splits) and
+//      above 2048 rows: T split where off-diagonals are negligible, for every
+//      block the smallest eigenvalues by multisection (bisection when there are
+//      many blocks) to LAPACK dstebz's default tolerance eps |T|, the k smallest
+//      overall kept, and their vectors by inverse iteration restricted to the
+//      block (LU with partial pivoting of T - lambda I), re-orthogonalised within
+//      clusters of close eigenvalues (modified Gram-Schmidt), stopped as LAPACK's
+//      dstein once the growth shows a rounding-level residual;
+//   5. back-transformation v = Q y with the stored reflectors in compact-WY
+//      blocks of eight: a CTA a vector up to 2048 rows, one CTA above while Y and
+//      a block fit in shared memory, reflector by reflector beyond.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -1,6 +1,7 @@
-// Small dense linear algebra in one CTA (matrices in shared memory):
-// Cholesky, triangular solves and a parallel cyclic Jacobi eigensolver, and
-// on top of them the per-iteration "small step" of block LOBPCG.
+// Small dense linear algebra in one CTA (matrices in shared memory and
+// registers): Cholesky, a direct eigensolver of the wanted pairs, a parallel
+// cyclic Jacobi eigensolver for what that refuses, and on top of them the
+// per-iteration "small step" of block LOBPCG.
 //
 // LOBPCG small step (restatement of one iteration of the linfa-linalg 0.2
 // LOBPCG loop that src/solvers/lobpcg.rs:327-358 calls; algorithm of Knyazev,
@@ -1826,14 +1827,12 @@ __global__ void __launch_bounds__(ST) k_small_dense(const double* __restrict__ a
 
 }  // namespace
 
-// SPECTRAL_INIT_SMALL_STEP=cta keeps the multi-warp small step for every
-// width (the single-warp version is the default up to 16 columns); read on
-// every call, so one process can compare both.
-// SPECTRAL_INIT_SMALL_STEP = warp (a single warp running the shared-memory
-// routines, up to 16 columns) | reg (a single warp, register-resident
-// Rayleigh-Ritz, up to 16 columns); default: the 128-thread CTA, measured
-// fastest at n = 1M (FP64 solve 103 ms against 107 / 123 ms).  Read on every
-// launch, so one process can compare them.
+// SPECTRAL_INIT_SMALL_STEP, read on every launch so that one process can compare
+// them: serial (the CTA with one-thread-per-column triangular solves and the
+// Jacobi iteration over all pairs), warp (one warp running the shared-memory
+// routines, up to 16 columns), reg (one warp, register-resident Rayleigh-Ritz, up
+// to 16 columns); anything else, or unset: the CTA with the direct pairs, 22 us a
+// step at 12 x 12 where the others take 49 and more.
 int small_step_variant() {
   const char* e = std::getenv("SPECTRAL_INIT_SMALL_STEP");
   if (e == nullptr) return 1;
@@ -1860,11 +1859,8 @@ void small_step_dev(const Exec& ex, LobpcgCtrl* ctrl, const double* gram, int ns
                                  static_cast<int>(smem)));
     attr_set[ex.device] = true;
   }
-  // the Rayleigh-Ritz problem has up to ns * m rows: up to 16 fit one warp's
-  // registers; wider blocks get a CTA, the widest the most threads
-  // (SPECTRAL_INIT_SMALL_STEP: unset, the CTA with the parallel Rayleigh-Ritz;
-  // serial, the CTA with one-thread-per-column triangular solves; warp / reg,
-  // one warp)
+  // the Rayleigh-Ritz problem has up to ns * m rows; above 24 the CTA gets 512
+  // threads (the one-warp variants take up to 16)
   const int variant = small_step_variant();
   const bool par = variant != 3;
   auto launch = [&](auto kernel, int threads) {
