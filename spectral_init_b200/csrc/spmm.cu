@@ -1501,7 +1501,10 @@ std::mutex g_tune_mu;
 std::map<TuneKey, int> g_tune;
 constexpr int64_t kTuneMinNnz = int64_t(1) << 22;  // operators the autotuner times
 constexpr int64_t kSlicedMinNnz = int64_t(1) << 21;  // operators whose rule may ask for the sliced kernels
-constexpr int64_t kLongestMinNnz = int64_t(1) << 18;  // operators whose longest row is looked for
+// Operators whose longest row is looked for: the look costs 20 to 30 us, the
+// synchronisation most of it, so plans from the first on, solves (milliseconds)
+// from the second, single products (32 us with 0.3 M entries) never.
+constexpr int64_t kLongestPlanNnz = int64_t(1) << 18, kLongestSolveNnz = int64_t(1) << 20;
 
 double mean_row(const OpDev& op) { return op.n > 0 ? static_cast<double>(op.nnz) / static_cast<double>(op.n) : 0.0; }
 
@@ -1830,7 +1833,7 @@ void attach_ruled(const Exec& ex, OpDev& op, RowBlocks& rb, bool sell_ok) {
   if (timed || forced) make_row_blocks(ex, op, rb);
   rb.sell_ok = sell_ok;
   rb.ruled = !timed;
-  if (op.nnz >= kLongestMinNnz) rb.longest = longest_row(ex, op);
+  if (sell_ok && op.nnz >= (rb.sell_outlives ? kLongestPlanNnz : kLongestSolveNnz)) rb.longest = longest_row(ex, op);
   rb.attach(op);
 }
 
