@@ -373,9 +373,13 @@ def test_a_plan_holds_the_copies_that_it_uses(gpu_ctx, monkeypatch):
     """With little free memory (1 GiB, by a test seam) a prepared operator's
     sliced copy waits for the first product that the rule gives it: 16 f64
     columns leave it unbuilt, 4 build it, and destroying the plan frees it."""
+    import gc
+
     import torch
     from cuda.bindings import driver
     import spectral_init_b200 as si
+
+    gc.collect()  # operators of earlier tests give their copies back now
 
     def used():
         gpu_ctx.synchronize()
